@@ -1220,6 +1220,222 @@ RWD void ix_list_eval(const Params<T>& P, const DevState<T>& S, int c, const ISt
   }
 }
 
+// Two floats in one 64-bit register: the packed FP32 instructions of sm_100 (each half
+// rounded to nearest on its own, so a packed operation gives the two scalar results).
+struct F2 {
+  unsigned long long v;
+};
+RWD F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+RWD F2 f2(float x) { return f2(x, x); }
+RWD float f2_lo(F2 a) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+  return lo;
+}
+RWD float f2_hi(F2 a) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+  return hi;
+}
+RWD F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+RWD F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+RWD F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+RWD F2 dot2(F2 ax, F2 ay, F2 az, F2 bx, F2 by, F2 bz) { return fma2(az, bz, fma2(ay, by, mul2(ax, bx))); }
+
+RWD float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+RWD float div_ftz(float a, float b) {
+  float y;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+
+// gv -= a (x) b where ok holds.
+RWD void add_grad(Acc<float>& A, float ax, float ay, float az, float bx, float by, float bz, bool ok) {
+  asm("{\n\t.reg .pred p;\n\t"
+      "setp.ne.s32 p, %15, 0;\n\t"
+      "@p fma.rn.f32 %0, %9, %12, %0;\n\t"
+      "@p fma.rn.f32 %1, %9, %13, %1;\n\t"
+      "@p fma.rn.f32 %2, %9, %14, %2;\n\t"
+      "@p fma.rn.f32 %3, %10, %12, %3;\n\t"
+      "@p fma.rn.f32 %4, %10, %13, %4;\n\t"
+      "@p fma.rn.f32 %5, %10, %14, %5;\n\t"
+      "@p fma.rn.f32 %6, %11, %12, %6;\n\t"
+      "@p fma.rn.f32 %7, %11, %13, %7;\n\t"
+      "@p fma.rn.f32 %8, %11, %14, %8;\n\t}"
+      : "+f"(A.gv.xx), "+f"(A.gv.xy), "+f"(A.gv.xz), "+f"(A.gv.yx), "+f"(A.gv.yy), "+f"(A.gv.yz), "+f"(A.gv.zx),
+        "+f"(A.gv.zy), "+f"(A.gv.zz)
+      : "f"(-ax), "f"(-ay), "f"(-az), "f"(bx), "f"(by), "f"(bz), "r"((int)ok));
+}
+// accden += rho dvk, s += f m where ok holds; av += g w where visc holds.
+RWD void add_force(Acc<float>& A, float rho, float dvk, float fx, float fy, float fz, float m, float gx, float gy,
+                   float gz, float w, bool ok, bool visc) {
+  asm("{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.s32 p, %17, 0;\n\t"
+      "setp.ne.s32 q, %18, 0;\n\t"
+      "@p fma.rn.f32 %0, %7, %8, %0;\n\t"
+      "@p fma.rn.f32 %1, %9, %12, %1;\n\t"
+      "@p fma.rn.f32 %2, %10, %12, %2;\n\t"
+      "@p fma.rn.f32 %3, %11, %12, %3;\n\t"
+      "@q fma.rn.f32 %4, %13, %16, %4;\n\t"
+      "@q fma.rn.f32 %5, %14, %16, %5;\n\t"
+      "@q fma.rn.f32 %6, %15, %16, %6;\n\t}"
+      : "+f"(A.accden), "+f"(A.s.x), "+f"(A.s.y), "+f"(A.s.z), "+f"(A.av.x), "+f"(A.av.y), "+f"(A.av.z)
+      : "f"(rho), "f"(dvk), "f"(fx), "f"(fy), "f"(fz), "f"(m), "f"(gx), "f"(gy), "f"(gz), "f"(w), "r"((int)ok),
+        "r"((int)visc));
+}
+
+// A neighbour record as its two 32-byte halves, in the order this lane reads them.
+struct RawRec {
+  float a[8], b[8];
+};
+RWD void load_half(const float* q, float (&v)[8]) {
+  asm
+  ("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(q));
+}
+
+// ix_list_eval<false, float, true> for the walk kernel, two entries at a time.  The terms
+// of the two pairs are formed by packed instructions (the same operations in the same
+// order as pair_eval<false>, each half rounded on its own); the sums take the entries one
+// after the other, so every sum is the one ix_list_eval forms, bit for bit.  Squares that
+// are then added stay scalar: the compiler fuses a packed multiply into a packed add.
+//
+// What bounds it: issue (half the cycles) and the L1 data stage (70% of its wavefronts)
+// together.  The stage serves two lanes' 32-byte sectors per cycle when they lie in
+// different halves of a line's 64-byte half, one otherwise (measured on random records:
+// 51 cycles per warp and record pair of loads, 33 when odd lanes read the halves in the
+// other order).  So odd lanes read the second half first, and the selects that put the
+// halves back in order are the moves that pair the two records' fields.  Packing halves
+// the issue slots of the pair terms; the packed instructions run at the FMA pipe's scalar
+// rate.  1.92M-particle wall, per launch: 1.004 ms scalar, 0.955 ms packed with branches
+// around the sums, 0.909 ms with predicated sums and the flushing reciprocals.
+RWD void ix_walk_pairs(const Params<float>& P, const DevState<float>& S, const IState<float>& I, const unsigned* lst,
+                       int stride, int cnt, Acc<float>& A) {
+  if (cnt <= 0) return;
+  const float* __restrict__ rec = reinterpret_cast<const float*>(S.rec);
+  const bool odd = threadIdx.x & 1;
+  const int h0 = odd ? 8 : 0;
+  const int last = cnt - 1;
+  auto entry = [&](int e) { return __ldcs(lst + min(e, last) * stride); };
+  auto load = [&](unsigned ent) {
+    RawRec r;
+    const float* q = rec + (size_t)(ent & 0x7ffffffu) * 16;
+    load_half(q + h0, r.a);
+    load_half(q + (h0 ^ 8), r.b);
+    return r;
+  };
+  const F2 px = f2(I.pos.x), py = f2(I.pos.y), pz = f2(I.pos.z);
+  const F2 vx = f2(I.vel.x), vy = f2(I.vel.y), vz = f2(I.vel.z), rho_i = f2(I.rho);
+  const F2 sxx = f2(I.sor.xx), syy = f2(I.sor.yy), szz = f2(I.sor.zz), sxy = f2(I.sor.xy), sxz = f2(I.sor.xz),
+           syz = f2(I.sor.yz);
+  const F2 neg = f2(-1.0f), th = f2(P.two_h);
+  const bool visc_on = P.viscosity_type == 1, art_on = P.art_coef != 0.0f, still = I.shift == 1;
+  const bool ri_pos = I.ri > 0.0f;
+  unsigned e0 = entry(0), e1 = entry(1);
+  RawRec r0 = load(e0), r1 = load(e1);
+  unsigned n0 = entry(2), n1 = entry(3);
+#pragma unroll 1
+  for (int e = 0; e < cnt; e += 2) {
+    auto lo = [&](int k) { return f2(odd ? r0.b[k] : r0.a[k], odd ? r1.b[k] : r1.a[k]); };
+    auto hi = [&](int k) { return f2(odd ? r0.a[k] : r0.b[k], odd ? r1.a[k] : r1.b[k]); };
+    const F2 qx = lo(0), qy = lo(1), qz = lo(2), ux = lo(4), uy = lo(5), uz = lo(6), rho_j = lo(7);
+    const F2 mass = hi(0), svol = hi(1), jxx = hi(2), jyy = hi(3), jzz = hi(4), jxy = hi(5), jxz = hi(6), jyz = hi(7);
+    const unsigned c0 = e0 >> 27, c1 = e1 >> 27;
+    e0 = n0;
+    e1 = n1;
+    r0 = load(e0);
+    r1 = load(e1);
+    n0 = entry(e + 4);
+    n1 = entry(e + 5);
+    // dr = (pos_i - p_j) - offset 2h, the offset digits of c = dx + 3 dy + 9 dz decoded as
+    // 1 - d (each exact, the product exact, one rounding)
+    const int z0 = (c0 * 57) >> 9, s0 = c0 - 9 * z0, y0 = (s0 * 11) >> 5, x0 = s0 - 3 * y0;
+    const int z1 = (c1 * 57) >> 9, s1 = c1 - 9 * z1, y1 = (s1 * 11) >> 5, x1 = s1 - 3 * y1;
+    auto digit = [&](int d0, int d1) {
+      return add2(f2(__int_as_float(0x4B400001 - d0), __int_as_float(0x4B400001 - d1)), f2(-12582912.0f));
+    };
+    const F2 dx = fma2(digit(x0, x1), th, fma2(qx, neg, px));
+    const F2 dy = fma2(digit(y0, y1), th, fma2(qy, neg, py));
+    const F2 dz = fma2(digit(z0, z1), th, fma2(qz, neg, pz));
+    const float ra = pair_r2(f2_lo(dx), f2_lo(dy), f2_lo(dz)), rb = pair_r2(f2_hi(dx), f2_hi(dy), f2_hi(dz));
+    const F2 r2 = f2(ra, rb);
+    // r = r2 / sqrt(r2); below the floor, 2 - q is 2 as at r2 = 0
+    const float ma = f_max(ra, 1e-30f), mb = f_max(rb, 1e-30f);
+    const F2 r = f2(ma * rsqrt_ftz(ma), mb * rsqrt_ftz(mb));
+    const F2 q = mul2(r, f2(P.i_h));
+    const bool ok0 = f2_lo(q) < 2.0f, ok1 = f2_hi(q) < 2.0f && e + 1 < cnt;
+    const F2 t = fma2(q, neg, f2(2.0f));
+    const F2 dwdr = mul2(mul2(mul2(f2(P.kgrad), t), t), t);
+    const F2 gx = mul2(dx, dwdr), gy = mul2(dy, dwdr), gz = mul2(dz, dwdr);
+    const float v0 = f2_lo(svol), v1 = f2_hi(svol);
+    const bool con0 = v0 < 0.0f, con1 = v1 < 0.0f;
+    F2 wx = fma2(ux, neg, vx), wy = fma2(uy, neg, vy), wz = fma2(uz, neg, vz);
+    if (still) {  // no velocity difference against a contact wall
+      wx = f2(con0 ? 0.0f : f2_lo(wx), con1 ? 0.0f : f2_hi(wx));
+      wy = f2(con0 ? 0.0f : f2_lo(wy), con1 ? 0.0f : f2_hi(wy));
+      wz = f2(con0 ? 0.0f : f2_lo(wz), con1 ? 0.0f : f2_hi(wz));
+    }
+    const F2 vol = f2(f_abs(v0), f_abs(v1));
+    const F2 kx = mul2(gx, vol), ky = mul2(gy, vol), kz = mul2(gz, vol);
+    const F2 dvk = dot2(wx, wy, wz, kx, ky, kz);
+    const F2 txx = add2(sxx, jxx), tyy = add2(syy, jyy), tzz = add2(szz, jzz);
+    const F2 txy = add2(sxy, jxy), txz = add2(sxz, jxz), tyz = add2(syz, jyz);
+    const F2 fx = dot2(txx, txy, txz, gx, gy, gz);
+    const F2 fy = dot2(txy, tyy, tyz, gx, gy, gz);
+    const F2 fz = dot2(txz, tyz, tzz, gx, gy, gz);
+    const F2 vd = dot2(wx, wy, wz, dx, dy, dz);
+    const F2 num = mul2(f2(P.visc_k), vd);
+    const F2 den = mul2(add2(r2, f2(P.eta)), mul2(f2(0.5f), add2(rho_i, rho_j)));
+    const F2 artv = f2(f2_lo(vd) < 0.0f ? div_ftz(f2_lo(num), f2_lo(den)) : 0.0f,
+                       f2_hi(vd) < 0.0f ? div_ftz(f2_hi(num), f2_hi(den)) : 0.0f);
+    const F2 mv = mul2(mass, artv);
+    const F2 tr = add2(add2(jxx, jyy), jzz);
+    // the sums of one pair, predicated instead of branched over (a lane or two of a warp
+    // usually has a candidate between 2h and the list radius)
+    auto sums = [&](auto half, bool ok, bool con) {
+      add_grad(A, half(wx), half(wy), half(wz), half(kx), half(ky), half(kz), ok);
+      add_force(A, I.rho, half(dvk), half(fx), half(fy), half(fz), half(mass), half(gx), half(gy), half(gz),
+                half(mv), ok && !con, ok && !con && visc_on);
+      if (art_on && ok && !con && (ri_pos || half(tr) > 0.0f)) {  // artificial stress, as in pair_eval
+        float rj = half(tr);
+        rj = rj > 0.0f ? __fmul_rn(rj, P.art_coef) : 0.0f;
+        float artp = I.ri + rj;
+        if (artp > 0.0f) {
+          const float ker = kernel_w(P.knorm, half(q));
+          artp = __fmul_rn(artp, f_pow(ker / P.kernel_dr, P.kernel_zero / P.kernel_dr));
+          const float w = __fmul_rn(half(mass), artp);
+          A.as.x = f_fma(-half(gx), w, A.as.x);
+          A.as.y = f_fma(-half(gy), w, A.as.y);
+          A.as.z = f_fma(-half(gz), w, A.as.z);
+        }
+      }
+    };
+    sums([](F2 v) { return f2_lo(v); }, ok0, con0);
+    sums([](F2 v) { return f2_hi(v); }, ok1, con1);
+  }
+}
+
 // Pair sums of particle i straight from global memory: phase 1 lists candidates in
 // shared memory (my[k * stride]), phase 2 evaluates them in order.  A list that fills
 // up is evaluated and emptied, and the scan resumes (order preserved).
@@ -1573,11 +1789,11 @@ template <class T> __global__ void __launch_bounds__(256) k_rebuild_lists(const 
 //    registers;
 //  - scan (Walk = false): scans the 27 cells for the particles without a list (lists
 //    off, or a list that overflowed) and carries the contact state of deleted slots.
-#ifndef RW_WALK_MIN_BLOCKS
-#define RW_WALK_MIN_BLOCKS 0  // resident blocks per SM the walk kernel's register budget aims at (0: none)
-#endif
+// The packed walk holds two records ahead and two in use: 128 registers, four blocks of
+// 128 threads per SM (five blocks spill: 1.83 ms per launch against 0.91).
+template <class T, bool Strict> constexpr bool kPackedWalk = !Strict && sizeof(T) == 4;
 template <class T, bool Strict, bool Walk>
-__global__ void __launch_bounds__(Walk ? IX_WALK_MAX_THREADS : IX_THREADS, Walk ? RW_WALK_MIN_BLOCKS : 0)
+__global__ void __launch_bounds__(Walk ? IX_WALK_MAX_THREADS : IX_THREADS, Walk && kPackedWalk<T, Strict> ? 4 : 0)
     k_interaction(const Params<T> P, DevState<T> S, const Dyn<T>* dyn, int cpar) {
   extern __shared__ unsigned nbl[];  // IX_CAP x blockDim, column per thread (scan only)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1604,7 +1820,8 @@ __global__ void __launch_bounds__(Walk ? IX_WALK_MAX_THREADS : IX_THREADS, Walk 
   IState<T> I;
   Acc<T> A;
   ix_begin<Strict>(P, S, c, i, cv, I, A);
-  if (Walk) ix_list_eval<Strict, T, true>(P, S, c, I, S.nbg[lb] + t, S.nbg_stride, kept, A);
+  if constexpr (Walk && kPackedWalk<T, Strict>) ix_walk_pairs(P, S, I, S.nbg[lb] + t, S.nbg_stride, kept, A);
+  else if (Walk) ix_list_eval<Strict, T, true>(P, S, c, I, S.nbg[lb] + t, S.nbg_stride, kept, A);
   else ix_sums_global<Strict>(P, S, c, celli, I, nbl + threadIdx.x, blockDim.x, IX_CAP, A);
   if (P.periodbound) ix_period<Strict>(P, S, c, i, celli, I, A);
   ix_finish<Strict>(P, S, c, cpar, i, celli, I, A, cv);

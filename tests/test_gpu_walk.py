@@ -1,0 +1,75 @@
+"""The packed walk of the interaction (two list entries at a time, predicated sums) against
+the chunked kernel, which evaluates every pair by itself with scalar instructions: every sum
+is the same, so the states agree bit for bit."""
+import numpy as np
+import pytest
+
+from retainwall_code_b200 import LoquatSph, _abi, cases as C
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ["pospres", "velrhop", "str", "accad", "acestn", "spin", "contact_mag", "contact_var"]
+
+
+def _tension():
+    """Stresses in tension: the artificial stress of both particles of a pair."""
+    c = C.column_collapse(5, 4, 6, seed=3, model="dp")
+    c.stress[c.npb:] *= np.where(np.arange(c.npm) % 3, 1.0, -0.5)[:, None]
+    c.velrhop[c.npb:, :3] = np.random.default_rng(3).uniform(-0.05, 0.05, (c.npm, 3))
+    return c
+
+
+def _coincident():
+    """Two pairs of particles at one place (r = 0), and one particle a rounding apart."""
+    c = C.column_collapse(6, 5, 7, seed=4)
+    p = c.pospres[c.npb:]
+    p[11, :3] = p[10, :3]
+    p[40, :3] = p[41, :3]
+    p[40, 0] = np.nextafter(np.float32(p[41, 0]), np.float32(1.0))
+    return c
+
+
+def _not_finite():
+    """A velocity and a stress that are not finite reach their neighbours within 2h only."""
+    c = C.column_collapse(9, 9, 9, seed=5)
+    c.velrhop[c.npb + 100, 0] = np.nan
+    c.stress[c.npb + 620, 2] = -np.inf
+    return c
+
+
+def _no_viscosity():
+    c = C.column_collapse(5, 5, 6, seed=6)
+    c.params["viscosity_type"] = 0
+    c.velrhop[c.npb:, :3] = np.random.default_rng(6).uniform(-0.05, 0.05, (c.npm, 3))
+    return c
+
+
+def _lone():
+    """Particles out of every other's reach beside a small column: lists of one entry."""
+    c = C.column_collapse(4, 4, 4, seed=7)
+    c.pospres[c.npb + 63, 2] += 0.02
+    c.pospres[c.npb + 60, 0] += 0.03
+    return c
+
+
+CASES = {
+    "tension": (_tension, 3), "coincident": (_coincident, 2), "not finite": (_not_finite, 1),
+    "no viscosity": (_no_viscosity, 5), "lone": (_lone, 5),
+    # contact against a wall that moves in (slide flags), lists of every length mod 4
+    "contact": (lambda: C.retaining_wall(nx=13, ny=7, nz=11, mode="passive", wall_speed=0.05, seed=8), 60),
+    "one": (lambda: C.column_collapse(1, 1, 1, seed=9), 4),
+}
+
+
+@pytest.mark.parametrize("skin", [0.02, 0.4])
+@pytest.mark.parametrize("name", CASES)
+def test_packed_walk_equals_single_pairs(name, skin):
+    make, steps = CASES[name]
+    a, b = LoquatSph(case=make()), LoquatSph(case=make())
+    a.set_option(_abi.OPT_LIST_SKIN, skin)
+    b.set_option(_abi.OPT_INTERACTION_KERNEL, 1)
+    a.step(steps)
+    b.step(steps)
+    for key in KEYS:
+        np.testing.assert_array_equal(a.get(key), b.get(key), err_msg=key)
+    assert a.list_stats()[1] == a.info().npm  # every particle walked a list
