@@ -374,7 +374,7 @@ template <class T> struct Engine final : EngineBase {
       // kept candidate lists, two buffers each (a list update after a permutation reads
       // one and writes the other), their displacement bounds, and the marked cells
       for (int b = 0; b < 2; ++b) {
-        if (lists_fit()) {  // list indices stay 32-bit
+        if (lists_fit()) {
           S.nbg[b] = dalloc<unsigned>((size_t)IX_CAP * (np - npb));
           S.nbg_cnt[b] = dalloc<int>(np - npb);
         }
@@ -965,7 +965,10 @@ template <class T> struct Engine final : EngineBase {
     o->integrator_threads = integ_threads;
   }
 
-  bool lists_fit() const { return (size_t)IX_CAP * (size_t)(P.np - P.npb) < ((size_t)1 << 31); }
+  // list indices stay 32-bit, and an entry holds 26 bits of particle index
+  bool lists_fit() const {
+    return (size_t)IX_CAP * (size_t)(P.np - P.npb) < ((size_t)1 << 31) && P.np < (int)kEntIdx;
+  }
   // Kept candidate lists: radius 2h + skin; all rebuilt once any particle may have moved
   // 0.45 skin since the last full build (two particles then close in by at most 0.9
   // skin, so every pair within 2h is still listed by a list built since).

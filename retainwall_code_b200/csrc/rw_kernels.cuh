@@ -81,8 +81,9 @@ template <class T> struct DevState {
   int* col_cnt;
   int* col_off;
   struct Chunk* chunks;
-  // Candidate lists of the soil particles (entry e of soil slot t at nbg[b][e * nbg_stride + t],
-  // encoded like the shared-memory lists), count per slot (-1: not kept).  Two buffers
+  // Candidate lists of the soil particles, four entries to a quad (entry e of soil slot t at
+  // nbg[b][(e / 4) * 4 * nbg_stride + 4 t + e % 4], the last quad filled up with an entry of
+  // the particle itself), count per slot (-1: not kept).  Two buffers
   // b, Dyn::lbuf the live one: a list update after a permutation reads the other.
   unsigned* nbg[2];
   int* nbg_cnt[2];
@@ -90,7 +91,7 @@ template <class T> struct DevState {
   // Per particle: bound on the distance moved since the last full build of the lists
   // (permuted with the particles, into the other buffer).
   float* dacc[2];
-  unsigned* nbb[2];  // boundary particles' kept lists (entry e of particle i at nbb[b][e * npb + i])
+  unsigned* nbb[2];  // boundary particles' kept lists, the same form with stride npb
   int* nbb_cnt[2];
   int* inv;          // inverse of the last permutation: new index of old index j
   int* queue;        // rows whose lists a list update rebuilds (Dyn::n_queue of them)
@@ -126,6 +127,47 @@ template <class T> RWD int key_of(const Params<T>& P, I3 c) {
   return c.x * P.cell_num[1] * P.cell_num[2] + c.y * P.cell_num[2] + c.z;
 }
 RWD I3 off_of(int oc) { return {oc % 3 - 1, (oc / 3) % 3 - 1, oc / 9 - 1}; }
+
+// Entry of a kept list: particle index in the low 26 bits, the digits dx, dy, dz (0..2) of
+// its cell's offset plus one in two bits each above them.  One shift and a mask per digit
+// give the offset (a digit of an offset number takes a multiply and two more operations),
+// which the walk pays per entry; lists are kept for np < 2^26 (lists_fit).
+constexpr unsigned kEntIdx = 0x3ffffffu;
+RWD unsigned list_entry(int j, int oc) {
+  return (unsigned)j | ((unsigned)(oc % 3) << 26) | ((unsigned)((oc / 3) % 3) << 28) | ((unsigned)(oc / 9) << 30);
+}
+RWD I3 entry_off(unsigned e) { return {(int)(e >> 26 & 3u) - 1, (int)(e >> 28 & 3u) - 1, (int)(e >> 30) - 1}; }
+// Quad q of the list of column t (lists of `stride` columns).
+RWD size_t quad_at(int q, size_t stride, int t) { return ((size_t)q * stride + t) * 4; }
+RWD uint4 load_quad(const unsigned* __restrict__ lists, int q, size_t stride, int t) {
+  return __ldcs(reinterpret_cast<const uint4*>(lists + quad_at(q, stride, t)));
+}
+// Entries of one list written in order, a quad at a time.
+struct QuadWriter {
+  unsigned* lists;
+  size_t stride;
+  int t, cnt = 0;
+  unsigned a = 0, b = 0, c = 0;
+  RWD void push(unsigned e, int cap) {
+    const int k = cnt & 3;
+    if (k == 3) {
+      if (cnt < cap) __stcs(reinterpret_cast<uint4*>(lists + quad_at(cnt >> 2, stride, t)), uint4{a, b, c, e});
+    } else {
+      if (k == 0) a = e;
+      else if (k == 1) b = e;
+      else c = e;
+    }
+    ++cnt;
+  }
+  // the last quad, filled up with `own` (any valid entry)
+  RWD void finish(unsigned own, int cap) {
+    const int k = cnt & 3;
+    if (k && cnt <= cap)
+      __stcs(reinterpret_cast<uint4*>(lists + quad_at(cnt >> 2, stride, t)),
+             uint4{a, k > 1 ? b : own, k > 2 ? c : own, own});
+  }
+};
+constexpr int kOwnCell = 13;  // offset number of a particle's own cell
 
 RWD float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 RWD float rmul(float a, float b) { return __fmul_rn(a, b); }
@@ -668,21 +710,20 @@ template <class T> RWD bool near_marked(const Params<T>& P, const DevState<T>& S
 // inside every cell whose particles all stayed).
 RWD void carry_list(const unsigned* __restrict__ src, const int* __restrict__ src_cnt, int o, unsigned* __restrict__ dst,
                     int* __restrict__ dst_cnt, int i, size_t stride, const int* __restrict__ inv) {
-  constexpr unsigned kIdx = 0x7ffffffu;  // entry: particle index in the low 27 bits
   const int cnt = src_cnt[o];
   dst_cnt[i] = cnt;
-  // eight entries at a time, their loads and index lookups issued together (a thread
-  // waits for two loads per eight entries, not two per entry)
-  for (int e0 = 0; e0 < cnt; e0 += 8) {
-    unsigned v[8];
-    int m[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = e0 + k < cnt ? __ldcs(src + (size_t)(e0 + k) * stride + o) : 0u;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) m[k] = e0 + k < cnt ? inv[v[k] & kIdx] : 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (e0 + k < cnt) __stcs(dst + (size_t)(e0 + k) * stride + i, (unsigned)m[k] | (v[k] & ~kIdx));
+  const int nq = (cnt + 3) >> 2;
+  // two quads at a time, their loads and index lookups issued together (a thread waits
+  // for two loads per eight entries, not two per entry)
+  auto map = [&](unsigned e) { return (unsigned)inv[e & kEntIdx] | (e & ~kEntIdx); };
+  auto put = [&](int q, uint4 v) { __stcs(reinterpret_cast<uint4*>(dst + quad_at(q, stride, i)), v); };
+  for (int q = 0; q < nq; q += 2) {
+    const bool two = q + 1 < nq;
+    uint4 v = load_quad(src, q, stride, o), w = two ? load_quad(src, q + 1, stride, o) : v;
+    v = uint4{map(v.x), map(v.y), map(v.z), map(v.w)};
+    w = uint4{map(w.x), map(w.y), map(w.z), map(w.w)};
+    put(q, v);
+    if (two) put(q + 1, w);
   }
 }
 
@@ -746,7 +787,7 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
   // The 27 cells in the reference's order; with `keep`, the candidates within the list
   // radius are recorded (same order) for later sections.
   auto scan = [&](const I3 cc, const V3<T> pp, bool keep) {
-    int cnt = 0;
+    QuadWriter out{nbb, (size_t)P.npb, i};
     for (int oc = 0; oc < 27; ++oc) {
       const I3 off = off_of(oc);
       const I3 cj{cc.x + off.x, cc.y + off.y, cc.z + off.z};
@@ -759,15 +800,15 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
           V3<T> dr = pp - ld3(pos, j);
           dr = dr - o;
           const T r2 = pair_r2(dr.x, dr.y, dr.z);
-          if (keep && r2 < P.r2_list) {
-            if (cnt < IX_CAP) nbb[(size_t)cnt * P.npb + i] = (unsigned)j | ((unsigned)oc << 27);
-            ++cnt;
-          }
+          if (keep && r2 < P.r2_list) out.push(list_entry(j, oc), IX_CAP);
           pair(j, dr, r2, mat_of(j));
         }
       }
     }
-    if (keep) S.nbb_cnt[lb][i] = cnt <= IX_CAP ? cnt : -1;
+    if (keep) {
+      out.finish(list_entry(i, kOwnCell), IX_CAP);
+      S.nbb_cnt[lb][i] = out.cnt <= IX_CAP ? out.cnt : -1;
+    }
   };
   const bool keep = S.nbb[0] && P.keep_lists;
   const int mode = keep ? dyn->ix_mode : 0;
@@ -781,10 +822,14 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
     // together and the next batch's entries loaded while it is in flight: a thread next
     // to the soil waits for about one load per four entries instead of a chain of loads
     // per entry.
-    constexpr unsigned kNone = 0x7ffffffu;  // index of no particle (np < 2^27)
+    constexpr unsigned kNone = kEntIdx;  // index of no particle (np < 2^26)
     auto entries = [&](int e0, unsigned* ent) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ent[k] = e0 + k < kept ? __ldcs(nbb + (size_t)(e0 + k) * P.npb + i) : kNone;
+      uint4 q{kNone, kNone, kNone, kNone};
+      if (e0 < kept) q = load_quad(nbb, e0 >> 2, (size_t)P.npb, i);
+      ent[0] = q.x;
+      ent[1] = e0 + 1 < kept ? q.y : kNone;
+      ent[2] = e0 + 2 < kept ? q.z : kNone;
+      ent[3] = e0 + 3 < kept ? q.w : kNone;
     };
     unsigned ent[4], nxt[4];
     entries(0, ent);
@@ -809,7 +854,7 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
         const int j = (int)(ent[k] & kNone);
         if (j == (int)kNone) continue;
         V3<T> dr = pos_i - V3<T>{pj[k].x, pj[k].y, pj[k].z};
-        dr = dr - mulI(off_of((int)(ent[k] >> 27)), th);
+        dr = dr - mulI(entry_off(ent[k]), th);
         pair(j, dr, pair_r2(dr.x, dr.y, dr.z), [&](V4<T>& v, T& m, S6<T>& s6) {
           v = vj[k];
           m = mj[k];
@@ -982,12 +1027,16 @@ template <class T> __global__ void __launch_bounds__(128) k_corner(const Params<
   const int kept = (S.nbg[0] && P.keep_lists && dyn->list_ok) ? S.nbg_cnt[dyn->lbuf][t] : -1;
   if (kept >= 0) {
     const Rec<T>* __restrict__ rec = S.rec;
-    const unsigned* __restrict__ lst = S.nbg[dyn->lbuf] + t;
+    const unsigned* __restrict__ lists = S.nbg[dyn->lbuf];
     const size_t stride = (size_t)S.nbg_stride;
-    constexpr unsigned kNone = 0x7ffffffu;  // index of no particle (np < 2^27)
+    constexpr unsigned kNone = kEntIdx;  // index of no particle (np < 2^26)
     auto entries = [&](int e0, unsigned* ent) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ent[k] = e0 + k < kept ? __ldcs(lst + (size_t)(e0 + k) * stride) : kNone;
+      uint4 q{kNone, kNone, kNone, kNone};
+      if (e0 < kept) q = load_quad(lists, e0 >> 2, stride, t);
+      ent[0] = q.x;
+      ent[1] = e0 + 1 < kept ? q.y : kNone;
+      ent[2] = e0 + 2 < kept ? q.z : kNone;
+      ent[3] = e0 + 3 < kept ? q.w : kNone;
     };
     unsigned ent[4], nxt[4];
     entries(0, ent);
@@ -1002,7 +1051,7 @@ template <class T> __global__ void __launch_bounds__(128) k_corner(const Params<
         const int j = (int)(ent[k] & kNone);
         if (j >= P.npb) continue;
         const NbVals<T>& b = nb[k];
-        visit(j, off_of((int)(ent[k] >> 27)), V3<T>{b.p.x, b.p.y, b.p.z}, [&] { return b.a.y < T(0); },
+        visit(j, entry_off(ent[k]), V3<T>{b.p.x, b.p.y, b.p.z}, [&] { return b.a.y < T(0); },
               [&] { return b.vr; });
       }
 #pragma unroll
@@ -1177,9 +1226,11 @@ template <class T> RWD T small_float(int v) {
   else return (T)v;
 }
 
-// Evaluates the listed candidates of particle i (entry k at my[k * stride]: index j |
-// cell offset << 27) in list order.  The cell offset is decoded arithmetically (no
-// table lookup, which would compete with the record gathers for the L1 data stage).
+// Evaluates listed candidates of particle i in list order: a kept list (quads of list
+// entries, `my` the list's first quad, `stride` columns) or the scan's shared-memory list
+// (entry k at my[k * stride]: index j | offset number << 27).  The cell offset is decoded
+// arithmetically (no table lookup, which would compete with the record gathers for the L1
+// data stage).
 template <bool Strict, class T, bool Kept = false>
 RWD void ix_list_eval(const Params<T>& P, const DevState<T>& S, int c, const IState<T>& I, const unsigned* my,
                       int stride, int cnt, Acc<T>& A) {
@@ -1188,29 +1239,37 @@ RWD void ix_list_eval(const Params<T>& P, const DevState<T>& S, int c, const ISt
   // Kept lists (global memory) are read once per interaction: streaming loads, so they
   // do not push the neighbour records out of L2.
   auto entry = [&](int k) -> unsigned {
-    if constexpr (Kept) return __ldcs(my + k);
-    else return my[k];
+    if constexpr (Kept) return __ldcs(my + quad_at(k >> 2, (size_t)stride, 0) + (k & 3));
+    else return my[k * stride];
   };
+  auto index = [](unsigned e) { return (int)(e & (Kept ? kEntIdx : 0x7ffffffu)); };
   // Entries are read two ahead and records one ahead, so a record's index is in hand
   // when its load is issued.
   unsigned ent = entry(0);
-  unsigned ent1 = cnt > 1 ? entry(stride) : 0u;
-  int oc = (int)(ent >> 27);
-  NbVals<T> nb = load_nb(rec, (int)(ent & 0x7ffffffu));
+  unsigned ent1 = cnt > 1 ? entry(1) : 0u;
+  unsigned oc = ent;
+  NbVals<T> nb = load_nb(rec, index(ent));
 #pragma unroll 2  // alternating record registers instead of copying the prefetched one
   for (int e = 0; e < cnt; ++e) {
     const NbVals<T> cur = nb;
-    const int occ = oc;
+    const unsigned occ = oc;
     if (e + 1 < cnt) {
-      oc = (int)(ent1 >> 27);
-      nb = load_nb(rec, (int)(ent1 & 0x7ffffffu));
-      if (e + 2 < cnt) ent1 = entry((e + 2) * stride);
+      oc = ent1;
+      nb = load_nb(rec, index(ent1));
+      if (e + 2 < cnt) ent1 = entry(e + 2);
     }
-    // cell offset digits of occ = dx + 3 dy + 9 dz (each 0..2), without a table
-    const int dz = (occ * 57) >> 9;
-    const int rr = occ - 9 * dz;
-    const int dy = (rr * 11) >> 5;
-    const int dx = rr - 3 * dy;
+    int dx, dy, dz;  // digits of the cell offset plus one (each 0..2)
+    if constexpr (Kept) {
+      dx = (int)(occ >> 26 & 3u);
+      dy = (int)(occ >> 28 & 3u);
+      dz = (int)(occ >> 30);
+    } else {
+      const int o = (int)(occ >> 27);
+      dz = (o * 57) >> 9;
+      const int rr = o - 9 * dz;
+      dy = (rr * 11) >> 5;
+      dx = rr - 3 * dy;
+    }
     const T th = P.two_h;
     // (pos_i - p_j) - (d - 1) 2h with one rounding after the exact product: the same
     // value as subtracting the tabulated offset
@@ -1329,20 +1388,25 @@ RWD void load_half(const float* q, float (&v)[8]) {
 // halves back in order are the moves that pair the two records' fields.  Packing halves
 // the issue slots of the pair terms; the packed instructions run at the FMA pipe's scalar
 // rate.  1.92M-particle wall, per launch: 1.004 ms scalar, 0.955 ms packed with branches
-// around the sums, 0.909 ms with predicated sums and the flushing reciprocals.
-RWD void ix_walk_pairs(const Params<float>& P, const DevState<float>& S, const IState<float>& I, const unsigned* lst,
-                       int stride, int cnt, Acc<float>& A) {
+// around the sums, 0.909 ms with predicated sums and the flushing reciprocals, 0.882 ms with
+// the lists in quads (two entries a load, digits of the offset by a mask).  Scalar terms on
+// the same lists: 0.903 ms (122 registers), 0.937 ms at five blocks.
+RWD void ix_walk_pairs(const Params<float>& P, const DevState<float>& S, const IState<float>& I,
+                       const unsigned* __restrict__ lists, int t_col, size_t stride, int cnt, Acc<float>& A) {
   if (cnt <= 0) return;
-  const float* __restrict__ rec = reinterpret_cast<const float*>(S.rec);
   const bool odd = threadIdx.x & 1;
-  const int h0 = odd ? 8 : 0;
-  const int last = cnt - 1;
-  auto entry = [&](int e) { return __ldcs(lst + min(e, last) * stride); };
+  const float* __restrict__ rec_a = reinterpret_cast<const float*>(S.rec) + (odd ? 8 : 0);
+  const float* __restrict__ rec_b = reinterpret_cast<const float*>(S.rec) + (odd ? 0 : 8);
+  const int last = (cnt - 1) & ~1;  // first entry of the last pair
+  auto entries = [&](int e) {
+    e = min(e, last);
+    return __ldcs(reinterpret_cast<const uint2*>(lists + quad_at(e >> 2, stride, t_col) + (e & 2)));
+  };
   auto load = [&](unsigned ent) {
     RawRec r;
-    const float* q = rec + (size_t)(ent & 0x7ffffffu) * 16;
-    load_half(q + h0, r.a);
-    load_half(q + (h0 ^ 8), r.b);
+    const size_t j = (size_t)(ent & kEntIdx) * 16;
+    load_half(rec_a + j, r.a);
+    load_half(rec_b + j, r.b);
     return r;
   };
   const F2 px = f2(I.pos.x), py = f2(I.pos.y), pz = f2(I.pos.z);
@@ -1352,32 +1416,30 @@ RWD void ix_walk_pairs(const Params<float>& P, const DevState<float>& S, const I
   const F2 neg = f2(-1.0f), th = f2(P.two_h);
   const bool visc_on = P.viscosity_type == 1, art_on = P.art_coef != 0.0f, still = I.shift == 1;
   const bool ri_pos = I.ri > 0.0f;
-  unsigned e0 = entry(0), e1 = entry(1);
-  RawRec r0 = load(e0), r1 = load(e1);
-  unsigned n0 = entry(2), n1 = entry(3);
+  // Entries two pairs ahead, records one pair ahead.
+  uint2 cur = entries(0), nxt = entries(2);
+  RawRec r0 = load(cur.x), r1 = load(cur.y);
 #pragma unroll 1
   for (int e = 0; e < cnt; e += 2) {
     auto lo = [&](int k) { return f2(odd ? r0.b[k] : r0.a[k], odd ? r1.b[k] : r1.a[k]); };
     auto hi = [&](int k) { return f2(odd ? r0.a[k] : r0.b[k], odd ? r1.a[k] : r1.b[k]); };
     const F2 qx = lo(0), qy = lo(1), qz = lo(2), ux = lo(4), uy = lo(5), uz = lo(6), rho_j = lo(7);
     const F2 mass = hi(0), svol = hi(1), jxx = hi(2), jyy = hi(3), jzz = hi(4), jxy = hi(5), jxz = hi(6), jyz = hi(7);
-    const unsigned c0 = e0 >> 27, c1 = e1 >> 27;
-    e0 = n0;
-    e1 = n1;
-    r0 = load(e0);
-    r1 = load(e1);
-    n0 = entry(e + 4);
-    n1 = entry(e + 5);
-    // dr = (pos_i - p_j) - offset 2h, the offset digits of c = dx + 3 dy + 9 dz decoded as
-    // 1 - d (each exact, the product exact, one rounding)
-    const int z0 = (c0 * 57) >> 9, s0 = c0 - 9 * z0, y0 = (s0 * 11) >> 5, x0 = s0 - 3 * y0;
-    const int z1 = (c1 * 57) >> 9, s1 = c1 - 9 * z1, y1 = (s1 * 11) >> 5, x1 = s1 - 3 * y1;
-    auto digit = [&](int d0, int d1) {
-      return add2(f2(__int_as_float(0x4B400001 - d0), __int_as_float(0x4B400001 - d1)), f2(-12582912.0f));
+    const unsigned c0 = cur.x >> 26, c1 = cur.y >> 26;
+    cur = nxt;
+    r0 = load(cur.x);
+    r1 = load(cur.y);
+    nxt = entries(e + 4);
+    // dr = (pos_i - p_j) - offset 2h.  A digit d masked in place (d << s) and or-ed into
+    // the bits of 3 2^22 is the float 3 2^22 + (d << s); one exact multiply-add makes it
+    // 1 - d, and the product with 2h is exact: one rounding.
+    auto digit = [&](unsigned mask, float scale) {
+      const F2 f = f2(__uint_as_float((c0 & mask) | 0x4B400000u), __uint_as_float((c1 & mask) | 0x4B400000u));
+      return fma2(f, f2(-scale), f2(12582912.0f * scale + 1.0f));
     };
-    const F2 dx = fma2(digit(x0, x1), th, fma2(qx, neg, px));
-    const F2 dy = fma2(digit(y0, y1), th, fma2(qy, neg, py));
-    const F2 dz = fma2(digit(z0, z1), th, fma2(qz, neg, pz));
+    const F2 dx = fma2(digit(3u, 1.0f), th, fma2(qx, neg, px));
+    const F2 dy = fma2(digit(12u, 0.25f), th, fma2(qy, neg, py));
+    const F2 dz = fma2(digit(48u, 0.0625f), th, fma2(qz, neg, pz));
     const float ra = pair_r2(f2_lo(dx), f2_lo(dy), f2_lo(dz)), rb = pair_r2(f2_hi(dx), f2_hi(dy), f2_hi(dz));
     const F2 r2 = f2(ra, rb);
     // r = r2 / sqrt(r2); below the floor, 2 - q is 2 as at r2 = 0
@@ -1651,13 +1713,13 @@ template <class T> __global__ void __launch_bounds__(256) k_build_lists(const Pa
   const V4<T>* __restrict__ pos = S.pos[c];
   const V3<T> pos_i = ld3(pos, i);
   const T th = P.two_h;
-  unsigned* __restrict__ out = S.nbg[lb] + t;
-  int cnt = 0;
+  QuadWriter out{S.nbg[lb], stride, t};
   for (int oc = 0; oc < 27; ++oc) {
     const I3 off = off_of(oc);
     const I3 cj{celli.x + off.x, celli.y + off.y, celli.z + off.z};
     if (!in_grid(P, cj)) continue;
     const int k = key_of(P, cj);
+    const unsigned code = list_entry(0, oc);
     const V3<T> pmo = pos_i - mulI(off, th);  // conservative pre-test only
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
@@ -1666,13 +1728,12 @@ template <class T> __global__ void __launch_bounds__(256) k_build_lists(const Pa
       for (int j = rg.x; j < rg.y; ++j) {
         const V4<T> pj = pos[j];
         const T dx = pmo.x - pj.x, dy = pmo.y - pj.y, dz = pmo.z - pj.z;
-        if (dx * dx + dy * dy + dz * dz < P.r2_list) {
-          if (cnt < IX_CAP) __stcs(out + (size_t)cnt * stride, (unsigned)j | ((unsigned)oc << 27));
-          ++cnt;
-        }
+        if (dx * dx + dy * dy + dz * dz < P.r2_list) out.push((unsigned)j | code, IX_CAP);
       }
     }
   }
+  out.finish(list_entry(i, kOwnCell), IX_CAP);
+  const int cnt = out.cnt;
   if (cnt > IX_CAP) {
     S.nbg_cnt[lb][t] = -1;
     atomicAdd(&dyn->n_spill, 1);
@@ -1745,7 +1806,8 @@ template <class T> __global__ void __launch_bounds__(256) k_rebuild_lists(const 
     if (lane == 0) beg[kSeg] = total;
     __syncwarp();
     const size_t stride = bnd ? (size_t)P.npb : (size_t)S.nbg_stride;
-    unsigned* __restrict__ out = bnd ? S.nbb[lb] + i : S.nbg[lb] + (i - P.npb);
+    unsigned* __restrict__ out = bnd ? S.nbb[lb] : S.nbg[lb];
+    const int col = bnd ? i : i - P.npb;
     int* __restrict__ count = bnd ? S.nbb_cnt[lb] + i : S.nbg_cnt[lb] + (i - P.npb);
     int cnt = 0;
     for (int b0 = 0; b0 < total; b0 += 32) {
@@ -1765,15 +1827,17 @@ template <class T> __global__ void __launch_bounds__(256) k_rebuild_lists(const 
         const V4<T> pj = pos[j];
         const T dx = pmo.x - pj.x, dy = pmo.y - pj.y, dz = pmo.z - pj.z;
         hit = dx * dx + dy * dy + dz * dz < P.r2_list;
-        ent = (unsigned)j | ((unsigned)oc << 27);
+        ent = list_entry(j, oc);
       }
       const unsigned bal = __ballot_sync(0xffffffffu, hit);
       if (hit) {
         const int e = cnt + __popc(bal & ((1u << lane) - 1u));
-        if (e < IX_CAP) __stcs(out + (size_t)e * stride, ent);
+        if (e < IX_CAP) __stcs(out + quad_at(e >> 2, stride, col) + (e & 3), ent);
       }
       cnt += __popc(bal);
     }
+    if (cnt < IX_CAP && lane < (-cnt & 3))  // fill up the last quad
+      __stcs(out + quad_at(cnt >> 2, stride, col) + (cnt & 3) + lane, list_entry(i, kOwnCell));
     if (lane == 0) {
       *count = cnt > IX_CAP ? -1 : cnt;  // an overflowed boundary list: Adami scans for it
       if (cnt > IX_CAP && !bnd) atomicAdd(&dyn->n_spill, 1);
@@ -1820,8 +1884,8 @@ __global__ void __launch_bounds__(Walk ? IX_WALK_MAX_THREADS : IX_THREADS, Walk 
   IState<T> I;
   Acc<T> A;
   ix_begin<Strict>(P, S, c, i, cv, I, A);
-  if constexpr (Walk && kPackedWalk<T, Strict>) ix_walk_pairs(P, S, I, S.nbg[lb] + t, S.nbg_stride, kept, A);
-  else if (Walk) ix_list_eval<Strict, T, true>(P, S, c, I, S.nbg[lb] + t, S.nbg_stride, kept, A);
+  if constexpr (Walk && kPackedWalk<T, Strict>) ix_walk_pairs(P, S, I, S.nbg[lb], t, (size_t)S.nbg_stride, kept, A);
+  else if (Walk) ix_list_eval<Strict, T, true>(P, S, c, I, S.nbg[lb] + (size_t)4 * t, S.nbg_stride, kept, A);
   else ix_sums_global<Strict>(P, S, c, celli, I, nbl + threadIdx.x, blockDim.x, IX_CAP, A);
   if (P.periodbound) ix_period<Strict>(P, S, c, i, celli, I, A);
   ix_finish<Strict>(P, S, c, cpar, i, celli, I, A, cv);
@@ -2372,15 +2436,18 @@ template <class T> __global__ void __launch_bounds__(128) k_shepard(const Params
   const int kept = (only_filter_steps && S.nbg[0] && P.keep_lists && dyn->list_ok) ? S.nbg_cnt[dyn->lbuf][t] : -1;
   if (kept >= 0) {
     const Rec<T>* __restrict__ rec = S.rec;
-    const unsigned* __restrict__ lst = S.nbg[dyn->lbuf] + t;
+    const unsigned* __restrict__ lists = S.nbg[dyn->lbuf];
     const size_t stride = (size_t)S.nbg_stride;
-    constexpr unsigned kNone = 0x7ffffffu;
+    constexpr unsigned kNone = kEntIdx;
     for (int e0 = 0; e0 < kept; e0 += 4) {
       unsigned ent[4];
       NbVals<T> nb[4];
       S6<T> sj[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ent[k] = e0 + k < kept ? __ldcs(lst + (size_t)(e0 + k) * stride) : kNone;
+      const uint4 q = load_quad(lists, e0 >> 2, stride, t);
+      ent[0] = q.x;
+      ent[1] = e0 + 1 < kept ? q.y : kNone;
+      ent[2] = e0 + 2 < kept ? q.z : kNone;
+      ent[3] = e0 + 3 < kept ? q.w : kNone;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int j = (int)(ent[k] & kNone);
@@ -2393,7 +2460,7 @@ template <class T> __global__ void __launch_bounds__(128) k_shepard(const Params
         const int j = (int)(ent[k] & kNone);
         if (j == (int)kNone || j < P.npb) continue;
         V3<T> dr = pos_i - V3<T>{nb[k].p.x, nb[k].p.y, nb[k].p.z};
-        dr = dr - mulI(off_of((int)(ent[k] >> 27)), th);
+        dr = dr - mulI(entry_off(ent[k]), th);
         const T r2 = pair_r2(dr.x, dr.y, dr.z);
         if (!(r2 < P.r2_prefilter)) continue;
         T r = pair_r(r2);
