@@ -752,6 +752,19 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
   V4<T> rps{T(0), T(0), T(0), T(0)}, rvr{T(0), T(0), T(0), T(0)};
   V3<T> n_i{T(0), T(0), T(0)};
   const T th = P.two_h;
+  // The sums take their products by explicit fused multiply-adds, so the list walk and the
+  // scan add alike.
+  auto add_normal = [&](const V3<T> dr, T q) {
+    const V3<T> g = dr * kernel_f(P.kgrad, q);
+    n_i = V3<T>{f_fma(-g.x, P.vol_def, n_i.x), f_fma(-g.y, P.vol_def, n_i.y), f_fma(-g.z, P.vol_def, n_i.z)};
+  };
+  auto add_material = [&](const V3<T> dr, T ker, T kv, const V4<T>& v, T m, const S6<T>& s) {
+    rs = S6<T>{f_fma(s.xx, kv, rs.xx), f_fma(s.yy, kv, rs.yy), f_fma(s.zz, kv, rs.zz),
+               f_fma(s.xy, kv, rs.xy), f_fma(s.xz, kv, rs.xz), f_fma(s.yz, kv, rs.yz)};
+    const T km = ker * m;
+    rps = V4<T>{f_fma(dr.x, km, rps.x), f_fma(dr.y, km, rps.y), f_fma(dr.z, km, rps.z), add_rn(rps.w, kv)};
+    rvr = V4<T>{f_fma(v.x, kv, rvr.x), f_fma(v.y, kv, rvr.y), f_fma(v.z, kv, rvr.z), f_fma(v.w, kv, rvr.w)};
+  };
   // One neighbour j at dr = (pos_i - pos_j) - offset 2h: boundary j (contact walls
   // only) feeds the wall normal, material j the extrapolation sums.
   // mat(v, m, s) supplies material j's velocity-density, mass and stress.
@@ -761,20 +774,14 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
     const T q = r * P.i_h;
     if (!(q < T(2.0f))) return;
     if (j < P.npb) {
-      T dwdr = kernel_f(P.kgrad, q);
-      V3<T> gker = dr * dwdr;
-      n_i = n_i - gker * P.vol_def;
+      add_normal(dr, q);
     } else {
       T ker = kernel_w(P.knorm, q);
       V4<T> vj;
       T mj;
       S6<T> sj;
       mat(vj, mj, sj);
-      T vol_j = mj / vj.w;
-      T kv = ker * vol_j;
-      rs = rs + sj * kv;
-      rps = rps + v4(dr * (ker * mj), kv);
-      rvr = rvr + vj * kv;
+      add_material(dr, ker, rmul(ker, mj / vj.w), vj, mj, sj);
     }
   };
   auto mat_of = [&](int j) {
@@ -841,27 +848,34 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
       S6<T> sj[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int j = (int)(ent[k] & kNone);
-        if (j == (int)kNone) continue;
+        // no particle: the boundary particle itself, its term not added below
+        const int j = (ent[k] & kNone) == kNone ? i : (int)(ent[k] & kNone);
         pj[k] = pos[j];
-        if (j >= P.npb) {
-          vj[k] = vel[j];
-          mj[k] = idm[j].y;
-          sj[k] = ld6(sa, sb, j);
-        }
+        vj[k] = vel[j];
+        mj[k] = idm[j].y;
+        sj[k] = ld6(sa, sb, j);
       }
       entries(e0 + 4, nxt);
+      // The four kernels and volumes are formed side by side without a branch (square
+      // roots, divisions and the kernel's double products are long chains), then the sums
+      // take the entries in order (65 -> 60 us a launch on the 1.92M wall, 38 -> 36 at 335k).
+      V3<T> dr[4];
+      T q[4], ker[4], kv[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int j = (int)(ent[k] & kNone);
-        if (j == (int)kNone) continue;
-        V3<T> dr = pos_i - V3<T>{pj[k].x, pj[k].y, pj[k].z};
-        dr = dr - mulI(entry_off(ent[k]), th);
-        pair(j, dr, pair_r2(dr.x, dr.y, dr.z), [&](V4<T>& v, T& m, S6<T>& s6) {
-          v = vj[k];
-          m = mj[k];
-          s6 = sj[k];
-        });
+        dr[k] = pos_i - V3<T>{pj[k].x, pj[k].y, pj[k].z};
+        dr[k] = dr[k] - mulI(entry_off(ent[k]), th);
+        const T r2 = pair_r2(dr[k].x, dr[k].y, dr[k].z);
+        q[k] = pair_r(r2) * P.i_h;
+        if (!(r2 < P.r2_prefilter) || (ent[k] & kNone) == kNone) q[k] = T(2.0f);
+        ker[k] = kernel_w(P.knorm, q[k]);
+        kv[k] = rmul(ker[k], mj[k] / vj[k].w);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (!(q[k] < T(2.0f))) continue;
+        if ((int)(ent[k] & kNone) < P.npb) add_normal(dr[k], q[k]);
+        else add_material(dr[k], ker[k], kv[k], vj[k], mj[k], sj[k]);
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) ent[k] = nxt[k];
@@ -958,15 +972,23 @@ template <class T> __global__ void k_mark_dilate(const Params<T> P, DevState<T> 
   }
 }
 
-template <class T> __global__ void __launch_bounds__(128) k_corner(const Params<T> P, DevState<T> S, const Dyn<T>* dyn,
-                                                                  int cpar) {
+// a.x b.x + a.y b.y + a.z b.z with fused multiply-adds at fixed places.
+template <class T> RWD T dot_fma(const V3<T> a, const V3<T> b) {
+  return f_fma(a.z, b.z, f_fma(a.y, b.y, rmul(a.x, b.x)));
+}
+
+// Capacity of the corner search's list of wall candidates (entries per thread).
+constexpr int CORNER_THREADS = 128, CORNER_CAP = 32;
+template <class T>
+__global__ void __launch_bounds__(CORNER_THREADS) k_corner(const Params<T> P, DevState<T> S, const Dyn<T>* dyn,
+                                                           int cpar) {
+  __shared__ unsigned found_sm[CORNER_CAP][CORNER_THREADS];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int npm = dyn->npm;
   if (t >= npm) return;
   const int i = P.npb + t;
   const int c = dyn->cur_main;
   const V4<T>* __restrict__ pos = S.pos[c];
-  const V3<T> pos_i = ld3(pos, i);
   const int4 cp = S.cellpos[c][i];
   const I3 celli{cp.x, cp.y, cp.z};
   V4<T> cv = S.cv[cpar][i];
@@ -982,92 +1004,123 @@ template <class T> __global__ void __launch_bounds__(128) k_corner(const Params<
                 S.codes[c][i].x >= 10);
     return;
   }
+  const V3<T> pos_i = ld3(pos, i);
   cv.x = T(0.0f);
   cv.y = T(999);
   T d_ij = T(999);
   V4<T> ny = S.cny[i];
-  V4<T> vz = S.cvz[i];
+  int nearest = -1;
   const T th = P.two_h;
-  // One boundary candidate j at in-cell position pj, in the cell at offset off (the body
-  // of the reference's scan).  contact(): j belongs to a contact wall; vel_of(): its
-  // velocity.
-  auto visit = [&](int j, const I3 off, const V3<T> pj, auto&& contact, auto&& vel_of) {
-    V3<T> dr = pos_i - pj - mulI(off, th);
-    const T r2 = pair_r2(dr.x, dr.y, dr.z);
-    if (!(r2 < P.r2_prefilter)) return;
-    T r = pair_r(r2);
-    T q = r * P.i_h;
-    if (!((double)q < 2.0)) return;
-    if (!contact()) return;
+  // One contact-wall candidate j at distance r = |dr|, q < 2, with normal n4 (the body of
+  // the reference's scan); the nearest one's wall and velocity are read at the end.
+  auto visit = [&](int j, const V3<T> dr, T r, T q, const V4<T>& n4) {
     T dwdr = kernel_f(P.kgrad, q);
     V3<T> gker = dr * dwdr;
     if (r < d_ij && r > T(0)) {
-      const V4<T> na4 = S.cny[j];
-      const V3<T> n_ad{na4.x, na4.y, na4.z};
+      const V3<T> n_ad{n4.x, n4.y, n4.z};
       const V3<T> n_mat = dr / r;
       d_ij = r;
-      cv.y = f_abs(dot(dr, n_ad));
-      cv.w = (T)S.codes[c][j].x;
-      const V4<T> vj = vel_of();
-      vz = V4<T>{vj.x, vj.y, vj.z, T(0)};
+      cv.y = f_abs(f_fma(dr.z, n_ad.z, f_fma(dr.x, n_ad.x, rmul(dr.y, n_ad.y))));
+      nearest = j;
       const T cos_c = T(0.866f);
-      const T cos_n = f_abs(dot(n_mat, n_ad));
+      const T cos_n = f_abs(dot_fma(n_mat, n_ad));
       if (cos_n < cos_c) ny = V4<T>{n_mat.x, n_mat.y, n_mat.z, T(0)};
       else ny = V4<T>{n_ad.x, n_ad.y, n_ad.z, T(0)};
     }
-    cv.x += f_abs((ny.x * gker.x + ny.y * gker.y + ny.z * gker.z) * P.vol_def);
+    cv.x += f_abs(rmul(dot_fma(xyz(ny), gker), P.vol_def));
+  };
+  auto offset_from = [&](const V4<T>& pj, const I3 off) {
+    return pos_i - V3<T>{pj.x, pj.y, pj.z} - mulI(off, th);
   };
   // The candidate lists, current once the search has built, updated or kept them
   // (list_ok), hold every boundary particle within 2h of i in the scan's order (per cell
   // offset, the boundary range first, ascending index): walking their boundary entries
   // visits the same candidates that pass the q < 2 test, in the same order, without the
   // boundary cells' full ranges.  The boundary neighbour records (written by the Adami
-  // kernel earlier in the section) carry j's position, velocity and contact flag in one
-  // 64-byte line; entries are read four at a time and their records together, so a
-  // near-wall thread waits for two loads per four entries instead of a chain of loads
-  // per entry.
+  // kernel earlier in the section) carry j's position and contact flag.
+  //
+  // In two passes, because a warp's lanes meet their wall particles at different places of
+  // their lists: taking each entry as it comes, the whole warp runs the chain of the nearest
+  // particle (normal read, square root, divisions) for nearly every entry of 63 (38 us a
+  // launch on the 56k-particle wall against 23, 49 against 32 at 335k, 46 against 41 at 1.92M,
+  // where reading every particle's cell takes the rest).  The
+  // first pass only collects the contact-wall entries within reach, eight entries' records
+  // at a time; the second takes the lanes' collected entries side by side, at most some 30,
+  // the next one's position and normal loaded meanwhile.  A full collection is taken and
+  // emptied before the first pass goes on.
   const int kept = (S.nbg[0] && P.keep_lists && dyn->list_ok) ? S.nbg_cnt[dyn->lbuf][t] : -1;
-  if (kept >= 0) {
+  if (kept > 0) {
     const Rec<T>* __restrict__ rec = S.rec;
     const unsigned* __restrict__ lists = S.nbg[dyn->lbuf];
     const size_t stride = (size_t)S.nbg_stride;
-    constexpr unsigned kNone = kEntIdx;  // index of no particle (np < 2^26)
-    auto entries = [&](int e0, unsigned* ent) {
-      uint4 q{kNone, kNone, kNone, kNone};
-      if (e0 < kept) q = load_quad(lists, e0 >> 2, stride, t);
-      ent[0] = q.x;
-      ent[1] = e0 + 1 < kept ? q.y : kNone;
-      ent[2] = e0 + 2 < kept ? q.z : kNone;
-      ent[3] = e0 + 3 < kept ? q.w : kNone;
-    };
-    unsigned ent[4], nxt[4];
-    entries(0, ent);
-    for (int e0 = 0; e0 < kept; e0 += 4) {
-      NbVals<T> nb[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if ((int)(ent[k] & kNone) < P.npb) nb[k] = load_nb(rec, (int)(ent[k] & kNone));
-      entries(e0 + 4, nxt);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int j = (int)(ent[k] & kNone);
-        if (j >= P.npb) continue;
-        const NbVals<T>& b = nb[k];
-        visit(j, entry_off(ent[k]), V3<T>{b.p.x, b.p.y, b.p.z}, [&] { return b.a.y < T(0); },
-              [&] { return b.vr; });
+    unsigned* found = &found_sm[0][threadIdx.x];
+    int n = 0;
+    auto take = [&] {
+      V4<T> pj{T(0), T(0), T(0), T(0)}, n4 = pj;
+      auto fetch = [&](int k) {
+        const unsigned j = found[k * CORNER_THREADS] & kEntIdx;
+        pj = rec[j].p;
+        n4 = S.cny[j];
+      };
+      if (n > 0) fetch(0);
+      for (int k = 0; k < n; ++k) {
+        const unsigned ent = found[k * CORNER_THREADS];
+        const V3<T> dr = offset_from(pj, entry_off(ent));
+        const V4<T> nk = n4;
+        if (k + 1 < n) fetch(k + 1);
+        const T r = pair_r(pair_r2(dr.x, dr.y, dr.z)), q = r * P.i_h;
+        if ((double)q < 2.0) visit((int)(ent & kEntIdx), dr, r, q, nk);
       }
+      n = 0;
+    };
+    const int last_q = (kept - 1) >> 2;
+    uint4 u = load_quad(lists, 0, stride, t), v = load_quad(lists, min(1, last_q), stride, t);
+    for (int q0 = 0; q0 <= last_q; q0 += 2) {
+      const unsigned ent[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+      V4<T> pj[8];
+      T vol[8];
+      bool bnd[8];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) ent[k] = nxt[k];
+      for (int k = 0; k < 8; ++k) {
+        bnd[k] = 4 * q0 + k < kept && (int)(ent[k] & kEntIdx) < P.npb;
+        if (bnd[k]) {
+          pj[k] = rec[ent[k] & kEntIdx].p;
+          vol[k] = rec[ent[k] & kEntIdx].a.y;
+        }
+      }
+      u = load_quad(lists, min(q0 + 2, last_q), stride, t);
+      v = load_quad(lists, min(q0 + 3, last_q), stride, t);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const V3<T> dr = offset_from(pj[k], entry_off(ent[k]));
+        if (bnd[k] && pair_r2(dr.x, dr.y, dr.z) < P.r2_prefilter && vol[k] < T(0)) {
+          found[n * CORNER_THREADS] = ent[k];
+          ++n;
+        }
+      }
+      if (n > CORNER_CAP - 8) take();
     }
-  } else {
+    take();
+  } else if (kept < 0) {
     for (int oc = 0; oc < 27; ++oc) {
       const I3 off = off_of(oc);
       const I3 cj{celli.x + off.x, celli.y + off.y, celli.z + off.z};
       if (!in_grid(P, cj)) continue;
       const int2 rg = S.range[key_of(P, cj)];
-      for (int j = rg.x; j < rg.y; ++j)
-        visit(j, off, ld3(pos, j), [&] { return S.codes[c][j].x >= 10; }, [&] { return S.vel[c][j]; });
+      for (int j = rg.x; j < rg.y; ++j) {
+        const V3<T> dr = offset_from(pos[j], off);
+        const T r2 = pair_r2(dr.x, dr.y, dr.z);
+        if (!(r2 < P.r2_prefilter)) continue;
+        const T r = pair_r(r2), q = r * P.i_h;
+        if ((double)q < 2.0 && S.codes[c][j].x >= 10) visit(j, dr, r, q, S.cny[j]);
+      }
     }
+  }
+  V4<T> vz = S.cvz[i];
+  if (nearest >= 0) {
+    cv.w = (T)S.codes[c][nearest].x;
+    const V4<T> vj = S.vel[c][nearest];
+    vz = V4<T>{vj.x, vj.y, vj.z, T(0)};
   }
   S.cv[cpar][i] = cv;
   S.cny[i] = ny;
