@@ -118,6 +118,8 @@ template <class T> struct Engine final : EngineBase {
   std::future<SaveResult> pending_save;
   unsigned char* stage_h = nullptr;  // page-locked staging of a save's arrays
   size_t stage_bytes = 0;
+  unsigned char* d_export = nullptr;  // rows of an export put together on the device
+  size_t export_bytes = 0;
   bool graph_cond = false;  // the instantiated step graph has the gates
   cudaStream_t st_body = nullptr;
 
@@ -156,12 +158,6 @@ template <class T> struct Engine final : EngineBase {
   }
   template <class X> void up(X* d, const std::vector<X>& h) {
     if (!h.empty()) RW_CU(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(X), cudaMemcpyHostToDevice, st));
-  }
-  template <class X> std::vector<X> down(const X* d, size_t n) {
-    std::vector<X> h(n);
-    if (n) RW_CU(cudaMemcpyAsync(h.data(), d, n * sizeof(X), cudaMemcpyDeviceToHost, st));
-    RW_CU(cudaStreamSynchronize(st));
-    return h;
   }
   int* need_ptr() { return &d_dyn->need_sort; }
   Dyn<T> dyn_host() {
@@ -392,6 +388,8 @@ template <class T> struct Engine final : EngineBase {
       tab = dalloc<HypoC<T>>(kModelMax);
       d_clstats = dalloc<double>(4);
       d_count = dalloc<unsigned long long>(1);
+      export_bytes = std::min<size_t>(9 * sizeof(T) * np, 8u << 20);
+      d_export = dalloc<unsigned char>(export_bytes);
       d_dyn = dalloc<Dyn<T>>(1);
     };
     measuring = true;
@@ -1064,90 +1062,84 @@ template <class T> struct Engine final : EngineBase {
     return P.np;
   }
 
+  // Writes to every page of a large destination from several host threads: the page faults
+  // of new memory otherwise run on the one thread that copies (a 35 MB array in 5 ms; 20 ms
+  // through a temporary vector on one thread).  Page-locked slots were slower to make (3 to
+  // 60 ms) than they saved.
+  static void touch(void* dst, size_t bytes) {
+    constexpr size_t kPage = 4096, kPerThread = 2u << 20;
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t of = std::min(bytes / kPerThread, std::min<size_t>(hw, 8));
+    auto part = [=](size_t w) {
+      volatile unsigned char* p = static_cast<unsigned char*>(dst);
+      for (size_t k = bytes * w / of; k < bytes * (w + 1) / of; k += kPage) p[k] = 0;
+    };
+    std::vector<std::thread> th;
+    try {
+      for (size_t w = 1; w < of; ++w) th.emplace_back(part, w);
+    } catch (const std::system_error&) {  // the copy meets the other pages itself
+    }
+    if (of) part(0);
+    for (auto& x : th) x.join();
+  }
+
   int get_array(int which, void* dst, size_t bytes) override {
     if (which < 0 || which >= RW_ARR_COUNT_) return RW_EINVAL;
-    const size_t n = rows(which);
-    if (bytes != n * row_bytes(which)) {
-      err = "rw_get_array: expected " + std::to_string(n * row_bytes(which)) + " bytes";
+    const size_t n = rows(which), rb = row_bytes(which);
+    if (bytes != n * rb) {
+      err = "rw_get_array: expected " + std::to_string(n * rb) + " bytes";
       return RW_EINVAL;
     }
-    RW_CU(cudaStreamSynchronize(st));
     Dyn<T> d = dyn_host();
     const int c = d.cur_main, cn = d.cur_nrm, ci = d.cur_ini;
-    T* o = (T*)dst;
-    auto put4 = [&](const V4<T>* src) {
-      auto h = down(src, n);
-      std::memcpy(dst, h.data(), n * sizeof(V4<T>));
+    auto put = [&](const void* src) {  // rows stored as they are returned
+      if (n) RW_CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
     };
-    auto put6 = [&](const V4<T>* a, const V2<T>* b) {
-      auto ha = down(a, n);
-      auto hb = down(b, n);
-      for (size_t i = 0; i < n; ++i) {
-        o[6 * i + 0] = ha[i].x; o[6 * i + 1] = ha[i].y; o[6 * i + 2] = ha[i].z;
-        o[6 * i + 3] = ha[i].w; o[6 * i + 4] = hb[i].x; o[6 * i + 5] = hb[i].y;
+    auto put_rows = [&](auto row) {  // rows put together on the device, element by element
+      using E = decltype(row(size_t(0), 0));
+      const int cols = (int)(rb / sizeof(E));
+      const size_t step = export_bytes / rb;
+      for (size_t first = 0; first < n; first += step) {
+        const size_t m = std::min(step, n - first);
+        k_export<<<nblk((long)(m * cols), 256), 256, 0, st>>>(row, first, m * cols, cols, reinterpret_cast<E*>(d_export));
+        check_launch();
+        RW_CU(cudaMemcpyAsync(static_cast<unsigned char*>(dst) + first * rb, d_export, m * rb, cudaMemcpyDeviceToHost, st));
       }
     };
+    auto put6 = [&](const V4<T>* a, const V2<T>* b) { put_rows(Rows6<T>{a, b}); };
+    touch(dst, bytes);
     switch (which) {
-      case RW_ARR_CODES: { auto h = down(S.codes[c], n); std::memcpy(dst, h.data(), bytes); break; }
-      case RW_ARR_CELLPOS: { auto h = down(S.cellpos[c], n); std::memcpy(dst, h.data(), bytes); break; }
-      case RW_ARR_POSPRES: put4(S.pos[c]); break;
-      case RW_ARR_POSPRES_ORI: put4(S.pos_ori[c]); break;
-      case RW_ARR_VELRHOP: put4(S.vel[c]); break;
-      case RW_ARR_IDMASSIDX: put4(S.idm[c]); break;
+      case RW_ARR_CODES: put(S.codes[c]); break;
+      case RW_ARR_CELLPOS: put(S.cellpos[c]); break;
+      case RW_ARR_POSPRES: put(S.pos[c]); break;
+      case RW_ARR_POSPRES_ORI: put(S.pos_ori[c]); break;
+      case RW_ARR_VELRHOP: put(S.vel[c]); break;
+      case RW_ARR_IDMASSIDX: put(S.idm[c]); break;
       case RW_ARR_STR: put6(S.str_a[c], S.str_b[c]); break;
       case RW_ARR_STN: put6(S.stn_a[c], S.stn_b[c]); break;
-      case RW_ARR_NORMAL: put4(S.normal[cn]); break;
-      case RW_ARR_CONTACT_MAG: {
-        auto hf = down(S.cf[cpar], n);
-        auto hy = down(S.cny, n);
-        auto hz = down(S.cvz, n);
-        for (size_t i = 0; i < n; ++i) {
-          o[9 * i + 0] = hf[i].x; o[9 * i + 1] = hf[i].y; o[9 * i + 2] = hf[i].z;
-          o[9 * i + 3] = hy[i].x; o[9 * i + 4] = hy[i].y; o[9 * i + 5] = hy[i].z;
-          o[9 * i + 6] = hz[i].x; o[9 * i + 7] = hz[i].y; o[9 * i + 8] = hz[i].z;
-        }
-        break;
-      }
-      case RW_ARR_CONTACT_VAR: put4(S.cv[cpar]); break;
-      case RW_ARR_ACCAD: put4(S.accad); break;
-      case RW_ARR_SPIN: put4(S.spin); break;
+      case RW_ARR_NORMAL: put(S.normal[cn]); break;
+      case RW_ARR_CONTACT_MAG: put_rows(RowsContact<T>{S.cf[cpar], S.cny, S.cvz}); break;
+      case RW_ARR_CONTACT_VAR: put(S.cv[cpar]); break;
+      case RW_ARR_ACCAD: put(S.accad); break;
+      case RW_ARR_SPIN: put(S.spin); break;
       case RW_ARR_ACESTN: put6(S.ace_a, S.ace_b); break;
-      case RW_ARR_POSPRES_INI: put4(S.pos_ini[ci]); break;
-      case RW_ARR_VELRHOP_INI: put4(S.vel_ini[ci]); break;
+      case RW_ARR_POSPRES_INI: put(S.pos_ini[ci]); break;
+      case RW_ARR_VELRHOP_INI: put(S.vel_ini[ci]); break;
       case RW_ARR_STR_INI: put6(S.stri_a[ci], S.stri_b[ci]); break;
       case RW_ARR_STN_INI: put6(S.stni_a[ci], S.stni_b[ci]); break;
-      case RW_ARR_PART_IDX: {
-        int* oi = (int*)dst;
+      case RW_ARR_PART_IDX:
         if (d.need_sort) {
-          auto h = down(S.sperm, n);
-          std::memcpy(oi, h.data(), bytes);
+          put(S.sperm);
         } else {
+          int* oi = (int*)dst;
           for (size_t i = 0; i < n; ++i) oi[i] = (int)i;
         }
         break;
-      }
-      case RW_ARR_CELL_BEG: case RW_ARR_CELL_END: {
-        auto h = down(S.range, n);
-        int* oi = (int*)dst;
-        for (size_t k = 0; k < n; ++k) {
-          const bool occ = h[k].y > h[k].x;
-          oi[k] = occ ? (which == RW_ARR_CELL_BEG ? h[k].x : h[k].y) : -1;
-        }
-        break;
-      }
-      case RW_ARR_POS_ABS: {
-        auto hp = down(S.pos[c], n);
-        auto hc = down(S.cellpos[c], n);
-        for (size_t i = 0; i < n; ++i) {
-          o[4 * i + 0] = hp[i].x + (T)hc[i].x * P.two_h;
-          o[4 * i + 1] = hp[i].y + (T)hc[i].y * P.two_h;
-          o[4 * i + 2] = hp[i].z + (T)hc[i].z * P.two_h;
-          o[4 * i + 3] = hp[i].w;
-        }
-        break;
-      }
+      case RW_ARR_CELL_BEG: case RW_ARR_CELL_END: put_rows(RowsCell{S.range, which == RW_ARR_CELL_END}); break;
+      case RW_ARR_POS_ABS: put_rows(RowsPosAbs<T>{S.pos[c], S.cellpos[c], P.two_h}); break;
       default: return RW_EINVAL;
     }
+    RW_CU(cudaStreamSynchronize(st));
     return RW_OK;
   }
 
@@ -1443,15 +1435,6 @@ template <class T> struct Engine final : EngineBase {
     const SaveResult r = pending_save.get();
     if (r.rc) err = r.msg;
     return r.rc;
-  }
-  void get6_cache(std::vector<T>& o) {
-    const size_t n = P.np;
-    auto ha = down(S.tc_a, n);
-    auto hb = down(S.tc_b, n);
-    for (size_t i = 0; i < n; ++i) {
-      o[6 * i + 0] = ha[i].x; o[6 * i + 1] = ha[i].y; o[6 * i + 2] = ha[i].z;
-      o[6 * i + 3] = ha[i].w; o[6 * i + 4] = hb[i].x; o[6 * i + 5] = hb[i].y;
-    }
   }
 };
 

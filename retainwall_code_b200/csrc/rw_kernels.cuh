@@ -2699,6 +2699,45 @@ static __global__ void k_wall_force_final(double* wsum, int nblocks) {
   for (int k = 0; k < 3; ++k) wsum[3 * nblocks + k] = a[k];
 }
 
+// ---------------------------------------------------------------------------------
+// Export of arrays whose rows are not stored as the reference lays them out: element k of a
+// run of rows from `first`, written to page-locked host memory in order.
+// ---------------------------------------------------------------------------------
+template <class T> struct Rows6 {
+  const V4<T>* a;
+  const V2<T>* b;
+  RWD T operator()(size_t i, int k) const {
+    return k < 4 ? reinterpret_cast<const T*>(a + i)[k] : reinterpret_cast<const T*>(b + i)[k - 4];
+  }
+};
+template <class T> struct RowsContact {
+  const V4<T>*f, *n, *v;
+  RWD T operator()(size_t i, int k) const {
+    return reinterpret_cast<const T*>((k < 3 ? f : k < 6 ? n : v) + i)[k % 3];
+  }
+};
+struct RowsCell {
+  const int2* range;
+  bool end;
+  RWD int operator()(size_t i, int) const {
+    const int2 r = range[i];
+    return r.y > r.x ? (end ? r.y : r.x) : -1;
+  }
+};
+template <class T> struct RowsPosAbs {
+  const V4<T>* pos;
+  const int4* cell;
+  T two_h;
+  RWD T operator()(size_t i, int k) const {
+    const T p = reinterpret_cast<const T*>(pos + i)[k];
+    return k < 3 ? add_rn(p, rmul((T)reinterpret_cast<const int*>(cell + i)[k], two_h)) : p;
+  }
+};
+template <class Row, class E> __global__ void k_export(Row row, size_t first, size_t n, int cols, E* out) {
+  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (k < n) out[k] = row(first + k / cols, (int)(k % cols));
+}
+
 // Totals of the kept candidate lists: out[0] += entries, out[1] += soil particles with a list.
 // Per-material constants of the hypoplastic update, once per case (rw_device.cuh).
 template <class T> __global__ void k_hypo_table(const Params<T> P, HypoC<T>* out) {

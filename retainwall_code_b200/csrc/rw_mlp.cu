@@ -411,6 +411,12 @@ struct rw_mlp {
   float* sx = nullptr;
   float* stg = nullptr;
   long long cap = 0, n = 0;
+  // Device copy of the host arrays of rw_mlp_forward / rw_mlp_grad, kept between calls up to
+  // kKeep bytes (a stream-ordered allocation goes back to the driver at each wait: 0.2 to
+  // 2 ms a call), larger ones allocated for the call.
+  static constexpr size_t kKeep = 64u << 20;
+  unsigned char* ws = nullptr;
+  size_t ws_bytes = 0;
   std::string msg;
   std::mutex mu;
 };
@@ -482,6 +488,41 @@ rw_status grad_dev(rw_mlp* m, const float* dx, const float* dt, long long n_all,
   MLP_CU(m, cudaGetLastError());
   return RW_OK;
 }
+
+// Device memory for one call (the caller holds the network's lock).
+struct CallBuffer {
+  rw_mlp* m;
+  unsigned char* p = nullptr;
+  bool own = false;
+  explicit CallBuffer(rw_mlp* net) : m(net) {}
+  rw_status get(size_t bytes) {
+    if (bytes <= m->ws_bytes) {
+      p = m->ws;
+      return RW_OK;
+    }
+    own = bytes > rw_mlp::kKeep;
+    if (!own && m->ws) {  // the last call's work was waited for
+      cudaFree(m->ws);
+      m->ws = nullptr;
+      m->ws_bytes = 0;
+    }
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return fail(m, RW_ECUDA, std::string("device memory of the call: ") + cudaGetErrorString(e));
+    }
+    if (!own) {
+      m->ws = p;
+      m->ws_bytes = bytes;
+    }
+    return RW_OK;
+  }
+  ~CallBuffer() {
+    cudaStreamSynchronize(m->st);  // nothing of the call is left on the buffer
+    if (own && p) cudaFree(p);
+  }
+};
 
 template <class F>
 rw_status guarded_mlp(rw_mlp* m, F&& f) {
@@ -561,7 +602,7 @@ rw_status rw_mlp_destroy(rw_mlp* m) {
   cudaSetDevice(m->device);
   if (m->st) cudaStreamSynchronize(m->st);
   for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->m, (void*)m->v, (void*)m->fw, (void*)m->bw,
-                  (void*)m->bias, (void*)m->err, (void*)m->loss, (void*)m->ranges, (void*)m->sx, (void*)m->stg})
+                  (void*)m->bias, (void*)m->err, (void*)m->loss, (void*)m->ranges, (void*)m->sx, (void*)m->stg, (void*)m->ws})
     if (p) cudaFree(p);
   if (m->st) cudaStreamDestroy(m->st);
   delete m;
@@ -595,18 +636,16 @@ rw_status rw_mlp_forward(rw_mlp* m, const float* x, int64_t n, float* y) {
   return guarded_mlp(m, [&]() -> rw_status {
     if (n < 0 || n > (1LL << 30) || (n > 0 && (!x || !y))) return fail(m, RW_EINVAL, "rw_mlp_forward: bad arguments");
     if (n == 0) return RW_OK;
-    float *dx = nullptr, *dy = nullptr;
-    MLP_CU(m, cudaMallocAsync((void**)&dx, (size_t)n * IN * sizeof(float), m->st));
-    MLP_CU(m, cudaMallocAsync((void**)&dy, (size_t)n * OUT * sizeof(float), m->st));
+    CallBuffer buf(m);
+    rw_status got = buf.get((size_t)n * (IN + OUT) * sizeof(float));
+    if (got != RW_OK) return got;
+    float *dx = reinterpret_cast<float*>(buf.p), *dy = dx + (size_t)n * IN;
     MLP_CU(m, cudaMemcpyAsync(dx, x, (size_t)n * IN * sizeof(float), cudaMemcpyHostToDevice, m->st));
     rw_status s = forward_dev(m, dx, (int)n, dy);
     if (s == RW_OK) {
       MLP_CU(m, cudaMemcpyAsync(y, dy, (size_t)n * OUT * sizeof(float), cudaMemcpyDeviceToHost, m->st));
       MLP_CU(m, cudaStreamSynchronize(m->st));
     }
-    cudaFreeAsync(dx, m->st);
-    cudaFreeAsync(dy, m->st);
-    cudaStreamSynchronize(m->st);
     return s;
   });
 }
@@ -614,9 +653,10 @@ rw_status rw_mlp_forward(rw_mlp* m, const float* x, int64_t n, float* y) {
 rw_status rw_mlp_grad(rw_mlp* m, const float* x, const float* t, int64_t n, double* loss, float* grad) {
   return guarded_mlp(m, [&]() -> rw_status {
     if (n <= 0 || n > (1LL << 30) || !x || !t || !grad) return fail(m, RW_EINVAL, "rw_mlp_grad: bad arguments");
-    float *dx = nullptr, *dt = nullptr;
-    MLP_CU(m, cudaMallocAsync((void**)&dx, (size_t)n * IN * sizeof(float), m->st));
-    MLP_CU(m, cudaMallocAsync((void**)&dt, (size_t)n * OUT * sizeof(float), m->st));
+    CallBuffer buf(m);
+    rw_status got = buf.get((size_t)n * (IN + OUT) * sizeof(float));
+    if (got != RW_OK) return got;
+    float *dx = reinterpret_cast<float*>(buf.p), *dt = dx + (size_t)n * IN;
     MLP_CU(m, cudaMemcpyAsync(dx, x, (size_t)n * IN * sizeof(float), cudaMemcpyHostToDevice, m->st));
     MLP_CU(m, cudaMemcpyAsync(dt, t, (size_t)n * OUT * sizeof(float), cudaMemcpyHostToDevice, m->st));
     MLP_CU(m, cudaMemsetAsync(m->grad, 0, NPARAM * sizeof(float), m->st));
@@ -632,9 +672,6 @@ rw_status rw_mlp_grad(rw_mlp* m, const float* x, const float* t, int64_t n, doub
       MLP_CU(m, cudaStreamSynchronize(m->st));
       if (loss) *loss = l / (double)(n * OUT);
     }
-    cudaFreeAsync(dx, m->st);
-    cudaFreeAsync(dt, m->st);
-    cudaStreamSynchronize(m->st);
     return s;
   });
 }

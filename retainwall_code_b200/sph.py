@@ -32,6 +32,7 @@ class LoquatSph:
             st = L.rw_create(project.encode(), device, precision, ct.byref(h))
         check(st, "rw_create", None)
         self._h = h
+        self._shape = self.info()  # particle and cell counts, scalar size: fixed with the context
         self.project = project
         self.precision = precision
 
@@ -163,13 +164,13 @@ class LoquatSph:
         return inf
 
     def get(self, name: str) -> np.ndarray:
-        rows, cols, dt = _abi.array_spec(name, self.info())
-        a = np.zeros((rows, cols), dt) if cols > 1 else np.zeros(rows, dt)
+        rows, cols, dt = _abi.array_spec(name, self._shape)
+        a = np.empty((rows, cols), dt) if cols > 1 else np.empty(rows, dt)
         self._c(lib().rw_get_array(self._h, _abi.ARRAYS[name], a.ctypes.data, a.nbytes), f"rw_get_array({name})")
         return a
 
     def set(self, name: str, a: np.ndarray) -> None:
-        rows, cols, dt = _abi.array_spec(name, self.info())
+        rows, cols, dt = _abi.array_spec(name, self._shape)
         a = np.ascontiguousarray(a, dtype=dt)
         self._c(lib().rw_set_array(self._h, _abi.ARRAYS[name], a.ctypes.data, a.nbytes), f"rw_set_array({name})")
 
