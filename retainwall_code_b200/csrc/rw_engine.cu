@@ -66,6 +66,9 @@ struct EngineBase {
   // Launches one whole step on this context's stream while that stream takes part in a
   // capture begun elsewhere (the batch's fork/join capture).
   virtual void launch_into_capture(bool gates) = 0;
+  // Particles of this case, and of all cases that the step being captured runs beside.
+  virtual void particles(long* soil, long* bnd) const = 0;
+  virtual void set_beside(long soil, long bnd) = 0;
   // Wall resultant computed on stream s into the device array d_out (3 doubles).
   virtual void wall_force_enqueue(cudaStream_t s, int mode, int wall_id, const double* strip, double* d_out) = 0;
   virtual cudaStream_t stream() const = 0;
@@ -516,12 +519,28 @@ template <class T> struct Engine final : EngineBase {
     if (lists_kept()) {
       gated([&](cudaGraphConditionalHandle h) { k_build_gate<T><<<1, 1, 0, st>>>(P, S, d_dyn, h); },
             [&] {
-              k_build_lists<T><<<nblk(P.np, 256), 256, 0, st>>>(P, S, d_dyn);
+              k_build_lists<T><<<nblk(P.np, 256), 256, 0, st>>>(P, S, d_dyn, adami_lanes() ? 1 : 0);
               k_rebuild_lists<T><<<4 * nsm, 256, 0, st>>>(P, S, d_dyn);
             });
       check_launch();
     }
   }
+  // Eight lanes per particle (see GroupRows) where a thread per particle leaves the GPU
+  // waiting: up to the sizes where the rows' shared-memory traffic costs what the shorter
+  // chain saves.  Counted over all cases that a batch runs side by side.  Walk, us a launch by
+  // thread / by eight lanes: FP32 28 / 15 at 693 particles, 32 / 19 at 5.4k, 43 / 41 at 20k,
+  // 36 / 41 at 28k; FP64 54 / 32 at 5.4k, 65 / 91 at 28k.  Adami, over boundary particles:
+  // FP32 28 / 17 at 16k, 31 / 22 at 28k, 31 / 28 at 43k, 36 / 47 at 85k; FP64 19 / 16 at 16k,
+  // 21 / 27 at 40k.
+  bool walk_lanes() const {
+    // the second pass over a periodic image runs on one lane of the eight
+    return !P.periodbound && std::max(beside_soil, (long)(P.np - P.npb)) <= (sizeof(T) == 4 ? 16384 : 12288);
+  }
+  bool adami_lanes() const {
+    return lists_kept() && S.nbb[0] && std::max(beside_bnd, (long)P.npb) <= (sizeof(T) == 4 ? 40960 : 16384);
+  }
+  long beside_soil = 0, beside_bnd = 0;  // particles of the batch being captured (0: this case alone)
+  // Soil candidate lists are kept only with the walk kernels.
   // Soil candidate lists are kept only with the walk kernels.
   bool lists_kept() const { return ix_kernel == 0 && P.np > P.npb && S.nbg[0] && P.keep_lists; }
   void search(int section) {
@@ -575,7 +594,10 @@ template <class T> struct Engine final : EngineBase {
   }
   void adami() override {
     if (P.npb == 0) return;
-    k_adami<T><<<nblk(P.npb, 128), 128, 0, st>>>(P, S, d_dyn);
+    if (adami_lanes())
+      k_adami_group<T><<<nblk((long)P.npb * kLanes, kGroupThreads), kGroupThreads, 0, st>>>(P, S, d_dyn);
+    else
+      k_adami<T><<<nblk(P.npb, 128), 128, 0, st>>>(P, S, d_dyn);
     check_launch();
   }
   void corner() override {
@@ -607,9 +629,14 @@ template <class T> struct Engine final : EngineBase {
                 if (strict_fp) k_interaction<T, true, false><<<g, IX_THREADS, sm1, st>>>(P, S, d_dyn, cpar);
                 else k_interaction<T, false, false><<<g, IX_THREADS, sm1, st>>>(P, S, d_dyn, cpar);
               });
-        const unsigned gw = nblk(n, walk_threads);
-        if (strict_fp) k_interaction<T, true, true><<<gw, walk_threads, 0, st>>>(P, S, d_dyn, cpar);
-        else k_interaction<T, false, true><<<gw, walk_threads, 0, st>>>(P, S, d_dyn, cpar);
+        // At most two blocks of 128 per SM: blocks of 64 fill the SMs more evenly (27,648
+        // particles are 216 blocks on 148 SMs; FP64 walk 66 -> 59 us, FP32 the same).
+        const int wt = nblk(n, 128) <= 2 * (unsigned)nsm ? std::min(walk_threads, 64) : walk_threads;
+        const unsigned gw = nblk(n, wt);
+        if (!strict_fp && lists_kept() && walk_lanes())
+          k_interaction_group<T><<<nblk((long)n * kLanes, wt), wt, 0, st>>>(P, S, d_dyn, cpar);
+        else if (strict_fp) k_interaction<T, true, true><<<gw, wt, 0, st>>>(P, S, d_dyn, cpar);
+        else k_interaction<T, false, true><<<gw, wt, 0, st>>>(P, S, d_dyn, cpar);
       }
       check_launch();
     }
@@ -875,6 +902,14 @@ template <class T> struct Engine final : EngineBase {
   }
 
   cudaGraph_t step_graph(bool gates) override { return capture_step(gates && graph_gates); }
+  void set_beside(long soil, long bnd) override {
+    beside_soil = soil;
+    beside_bnd = bnd;
+  }
+  void particles(long* soil, long* bnd) const override {
+    *soil = P.np - P.npb;
+    *bnd = P.npb;
+  }
   void launch_into_capture(bool gates) override {
     const int c0 = cpar;
     allow_cond = gates && graph_gates;
@@ -1508,7 +1543,21 @@ struct Batch {
   }
   void build() {
     generations.clear();
-    for (EngineBase* e : engines) generations.push_back(e->generation);
+    long soil = 0, bnd = 0;
+    for (EngineBase* e : engines) {
+      generations.push_back(e->generation);
+      long m = 0, b = 0;
+      e->particles(&m, &b);
+      soil += m;
+      bnd += b;
+    }
+    struct Beside {  // the contexts' own graphs are captured for one case again afterwards
+      std::vector<EngineBase*>& all;
+      ~Beside() {
+        for (EngineBase* e : all) e->set_beside(0, 0);
+      }
+    } beside{engines};
+    for (EngineBase* e : engines) e->set_beside(soil, bnd);
     if (build_forked()) return;
     for (int attempt = 0; attempt < 2 && !gexec; ++attempt) {
       const bool gates = attempt == 0;

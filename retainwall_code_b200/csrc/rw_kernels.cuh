@@ -730,8 +730,154 @@ RWD void carry_list(const unsigned* __restrict__ src, const int* __restrict__ sr
 }
 
 // ---------------------------------------------------------------------------------
+// Eight lanes per particle, for cases too small to fill the GPU with a thread per particle:
+// there a launch lasts as long as one thread's chain of list entries (two or three waits per
+// entry or pair of them, whatever the number of particles).  Here each lane forms the terms
+// of one entry of eight, and then every lane adds up to three of the particle's sums over the
+// eight entries in list order, from shared memory: each sum is still one chain of fused
+// multiply-adds over the list, so it is the sum one thread forms, bit for bit.
+// A row holds one entry's terms as five groups of four; a sum's lane multiplies one scalar of
+// the row (at x) with three (at y).
+// ---------------------------------------------------------------------------------
+constexpr int kLanes = 8, kGroupThreads = 128, kRow = 20;
+template <class T> struct GroupRows {
+  // two buffers: a row is read while the next round's are written; a warp's four particles
+  // lie 8 elements apart in their banks
+  V4<T> row[2][kGroupThreads / 32][4][(kLanes * kRow + 8) / 4];
+};
+// The lane's three sums over the rows of one round; bit k of `on`: entry k counts.
+template <class T> RWD void group_add(const V4<T>* rows, int x, int y, unsigned on, T (&acc)[3]) {
+  const T* r = reinterpret_cast<const T*>(rows);
+#pragma unroll
+  for (int k = 0; k < kLanes; ++k) {
+    const V4<T> v = *reinterpret_cast<const V4<T>*>(r + k * kRow + y);
+    const T f = r[k * kRow + x];
+    if (on >> k & 1u) {
+      acc[0] = f_fma(f, v.x, acc[0]);
+      acc[1] = f_fma(f, v.y, acc[1]);
+      acc[2] = f_fma(f, v.z, acc[2]);
+    }
+  }
+}
+RWD float from_lane(float v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+RWD double from_lane(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+// Entry e of the list of column t, or an entry of the particle itself past the end.
+RWD unsigned group_entry(const unsigned* __restrict__ lists, size_t stride, int t, int e, int cnt, unsigned own) {
+  return e < cnt ? __ldcs(lists + quad_at(e >> 2, stride, t) + (e & 3)) : own;
+}
+
+// ---------------------------------------------------------------------------------
 // Adami boundary (src/adami_boundary.cu:26-158).
 // ---------------------------------------------------------------------------------
+// End of the Adami kernel for boundary particle i: wall normal, extrapolated velocity and
+// stress, neighbour record.
+template <class T>
+RWD void adami_finish(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int c, int i, bool contact,
+                      const int4& code, const V3<T> pos_i, const I3 celli, const V3<T> n_i, const S6<T>& rs,
+                      const V4<T>& rps, const V4<T>& rvr) {
+  const V4<T>* __restrict__ vel = S.vel[c];
+  const T nn = f_sqrt(f_fma(n_i.z, n_i.z, f_fma(n_i.y, n_i.y, rmul(n_i.x, n_i.x))));
+  if (nn > T(0)) {
+    S.cny[i] = V4<T>{n_i.x / nn, n_i.y / nn, n_i.z / nn, T(0)};
+  }
+  V4<T> vr_out = vel[i];
+  S6<T> str_out;
+  if (rps.w > T(0.0f)) {
+    const T kersum = rps.w;
+    const V3<T> dr_ref = xyz(rps);
+    const V4<T> nrm4 = S.normal[dyn->cur_nrm][i];
+    const T fcoef = nrm4.w;
+    const V3<T> nrm = xyz(nrm4);
+    const V3<T> vel_ref = xyz(rvr) / kersum;
+    const V3<T> vel_ref_n = nrm * dot(nrm, vel_ref);
+    const V3<T> vel_ref_t = vel_ref - vel_ref_n;
+    V3<T> vel_rb{T(0.0f), T(0.0f), T(0.0f)};
+    if (code.y == 1) {
+      const Motion<T>& mv = dyn->mv[code.w];
+      vel_rb = V3<T>{mv.trans_vel.x, mv.trans_vel.y, mv.trans_vel.z};
+      if (mv.is_rotat) {
+        V3<T> pabs = pos_i + mulI(celli, T(2.0f) * P.h);
+        V3<T> rp{mv.pos_rp.x, mv.pos_rp.y, mv.pos_rp.z};
+        V3<T> w{mv.rotat_vel.x, mv.rotat_vel.y, mv.rotat_vel.z};
+        vel_rb = vel_rb + cross(w, pabs - rp);
+      }
+    }
+    const V3<T> vel_rb_n = nrm * dot(nrm, vel_rb);
+    const V3<T> vel_rb_t = vel_rb - vel_rb_n;
+    const V3<T> vel_ext_n = vel_rb_n * T(2.0f) - vel_ref_n;
+    const V3<T> vel_ext_t = fcoef == T(-1.0f) ? vel_rb_t * T(2.0f) - vel_ref_t : vel_ref_t;
+    const V3<T> vel_ext = vel_ext_n + vel_ext_t;
+    const T rho = rvr.w / kersum;
+    vr_out = v4(vel_ext, rho);
+    if (contact) {
+      vr_out = v4(vel_rb, rho);
+      S.cvz[i] = V4<T>{vel_ext.x, vel_ext.y, vel_ext.z, T(0)};
+    }
+    const S6<T> str_ref = rs / kersum;
+    const V3<T> g{P.gravity[0], P.gravity[1], P.gravity[2]};
+    str_out = subdiag(str_ref, (g * dr_ref) / kersum);
+    S.vel[c][i] = vr_out;
+  } else {
+    str_out = zero6<T>();
+  }
+  st6(S.str_a[c], S.str_b[c], i, str_out);
+  write_rec(P, S.rec, i, S.pos[c][i], vr_out, str_out, P.vol_def * vr_out.w, contact);
+}
+
+// Sums of one boundary particle.  The products are explicit fused multiply-adds, so the list
+// walks and the scan add alike.
+template <class T> struct AdamiSums {
+  S6<T> rs;        // stress
+  V4<T> rps, rvr;  // distance and kernel sum; velocity and density
+  V3<T> n_i;       // wall normal
+  RWD void add_normal(const Params<T>& P, const V3<T> dr, T q) {
+    const V3<T> g = dr * kernel_f(P.kgrad, q);
+    n_i = V3<T>{f_fma(-g.x, P.vol_def, n_i.x), f_fma(-g.y, P.vol_def, n_i.y), f_fma(-g.z, P.vol_def, n_i.z)};
+  }
+  RWD void add_material(const V3<T> dr, T ker, T kv, const V4<T>& v, T m, const S6<T>& s) {
+    rs = S6<T>{f_fma(s.xx, kv, rs.xx), f_fma(s.yy, kv, rs.yy), f_fma(s.zz, kv, rs.zz),
+               f_fma(s.xy, kv, rs.xy), f_fma(s.xz, kv, rs.xz), f_fma(s.yz, kv, rs.yz)};
+    const T km = ker * m;
+    rps = V4<T>{f_fma(dr.x, km, rps.x), f_fma(dr.y, km, rps.y), f_fma(dr.z, km, rps.z), add_rn(rps.w, kv)};
+    rvr = V4<T>{f_fma(v.x, kv, rvr.x), f_fma(v.y, kv, rvr.y), f_fma(v.z, kv, rvr.z), f_fma(v.w, kv, rvr.w)};
+  }
+};
+// Boundary particle i's neighbours in the 27 cells around cc, in the reference's order:
+// boundary ones (contact walls only) feed the wall normal, material ones the extrapolation
+// sums.  With `keep`, the candidates within the list radius are recorded (same order).
+template <class T>
+RWD void adami_scan(const Params<T>& P, const DevState<T>& S, int c, const I3 cc, const V3<T> pp, bool contact,
+                    AdamiSums<T>& A, QuadWriter* keep) {
+  const V4<T>* __restrict__ pos = S.pos[c];
+  for (int oc = 0; oc < 27; ++oc) {
+    const I3 off = off_of(oc);
+    const I3 cj{cc.x + off.x, cc.y + off.y, cc.z + off.z};
+    if (!in_grid(P, cj)) continue;
+    const int k = key_of(P, cj);
+    const V3<T> o = mulI(off, P.two_h);
+    for (int layer = contact ? 0 : 1; layer < 2; ++layer) {
+      const int2 rg = S.range[layer ? k + P.ncell_material : k];
+      for (int j = rg.x; j < rg.y; ++j) {
+        V3<T> dr = pp - ld3(pos, j);
+        dr = dr - o;
+        const T r2 = pair_r2(dr.x, dr.y, dr.z);
+        if (keep && r2 < P.r2_list) keep->push(list_entry(j, oc), IX_CAP);
+        if (!(r2 < P.r2_prefilter)) continue;  // conservative: q >= 2 beyond it
+        const T q = pair_r(r2) * P.i_h;
+        if (!(q < T(2.0f))) continue;
+        if (j < P.npb) {
+          A.add_normal(P, dr, q);
+        } else {
+          const T ker = kernel_w(P.knorm, q);
+          const V4<T> vj = S.vel[c][j];
+          const T mj = S.idm[c][j].y;
+          A.add_material(dr, ker, rmul(ker, mj / vj.w), vj, mj, ld6(S.str_a[c], S.str_b[c], j));
+        }
+      }
+    }
+  }
+}
+
 template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.npb) return;
@@ -748,77 +894,10 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
   const I3 celli{cp.x, cp.y, cp.z};
   const int4 code = S.codes[c][i];
   const bool contact = code.x >= 10;
-  S6<T> rs = zero6<T>();
-  V4<T> rps{T(0), T(0), T(0), T(0)}, rvr{T(0), T(0), T(0), T(0)};
-  V3<T> n_i{T(0), T(0), T(0)};
+  AdamiSums<T> A{zero6<T>(), V4<T>{T(0), T(0), T(0), T(0)}, V4<T>{T(0), T(0), T(0), T(0)}, V3<T>{T(0), T(0), T(0)}};
   const T th = P.two_h;
-  // The sums take their products by explicit fused multiply-adds, so the list walk and the
-  // scan add alike.
-  auto add_normal = [&](const V3<T> dr, T q) {
-    const V3<T> g = dr * kernel_f(P.kgrad, q);
-    n_i = V3<T>{f_fma(-g.x, P.vol_def, n_i.x), f_fma(-g.y, P.vol_def, n_i.y), f_fma(-g.z, P.vol_def, n_i.z)};
-  };
-  auto add_material = [&](const V3<T> dr, T ker, T kv, const V4<T>& v, T m, const S6<T>& s) {
-    rs = S6<T>{f_fma(s.xx, kv, rs.xx), f_fma(s.yy, kv, rs.yy), f_fma(s.zz, kv, rs.zz),
-               f_fma(s.xy, kv, rs.xy), f_fma(s.xz, kv, rs.xz), f_fma(s.yz, kv, rs.yz)};
-    const T km = ker * m;
-    rps = V4<T>{f_fma(dr.x, km, rps.x), f_fma(dr.y, km, rps.y), f_fma(dr.z, km, rps.z), add_rn(rps.w, kv)};
-    rvr = V4<T>{f_fma(v.x, kv, rvr.x), f_fma(v.y, kv, rvr.y), f_fma(v.z, kv, rvr.z), f_fma(v.w, kv, rvr.w)};
-  };
-  // One neighbour j at dr = (pos_i - pos_j) - offset 2h: boundary j (contact walls
-  // only) feeds the wall normal, material j the extrapolation sums.
-  // mat(v, m, s) supplies material j's velocity-density, mass and stress.
-  auto pair = [&](int j, const V3<T> dr, const T r2, auto&& mat) {
-    if (!(r2 < P.r2_prefilter)) return;  // conservative: q >= 2 beyond it
-    const T r = pair_r(r2);
-    const T q = r * P.i_h;
-    if (!(q < T(2.0f))) return;
-    if (j < P.npb) {
-      add_normal(dr, q);
-    } else {
-      T ker = kernel_w(P.knorm, q);
-      V4<T> vj;
-      T mj;
-      S6<T> sj;
-      mat(vj, mj, sj);
-      add_material(dr, ker, rmul(ker, mj / vj.w), vj, mj, sj);
-    }
-  };
-  auto mat_of = [&](int j) {
-    return [&, j](V4<T>& v, T& m, S6<T>& s) {
-      v = vel[j];
-      m = idm[j].y;
-      s = ld6(sa, sb, j);
-    };
-  };
   const int lb = dyn->lbuf;
   unsigned* __restrict__ nbb = S.nbb[lb];
-  // The 27 cells in the reference's order; with `keep`, the candidates within the list
-  // radius are recorded (same order) for later sections.
-  auto scan = [&](const I3 cc, const V3<T> pp, bool keep) {
-    QuadWriter out{nbb, (size_t)P.npb, i};
-    for (int oc = 0; oc < 27; ++oc) {
-      const I3 off = off_of(oc);
-      const I3 cj{cc.x + off.x, cc.y + off.y, cc.z + off.z};
-      if (!in_grid(P, cj)) continue;
-      const int k = key_of(P, cj);
-      const V3<T> o = mulI(off, th);
-      for (int layer = contact ? 0 : 1; layer < 2; ++layer) {
-        const int2 rg = S.range[layer ? k + P.ncell_material : k];
-        for (int j = rg.x; j < rg.y; ++j) {
-          V3<T> dr = pp - ld3(pos, j);
-          dr = dr - o;
-          const T r2 = pair_r2(dr.x, dr.y, dr.z);
-          if (keep && r2 < P.r2_list) out.push(list_entry(j, oc), IX_CAP);
-          pair(j, dr, r2, mat_of(j));
-        }
-      }
-    }
-    if (keep) {
-      out.finish(list_entry(i, kOwnCell), IX_CAP);
-      S.nbb_cnt[lb][i] = out.cnt <= IX_CAP ? out.cnt : -1;
-    }
-  };
   const bool keep = S.nbb[0] && P.keep_lists;
   const int mode = keep ? dyn->ix_mode : 0;
   // In a list update (mode 2) the lists next to a marked cell were rebuilt and the
@@ -874,66 +953,106 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         if (!(q[k] < T(2.0f))) continue;
-        if ((int)(ent[k] & kNone) < P.npb) add_normal(dr[k], q[k]);
-        else add_material(dr[k], ker[k], kv[k], vj[k], mj[k], sj[k]);
+        if ((int)(ent[k] & kNone) < P.npb) A.add_normal(P, dr[k], q[k]);
+        else A.add_material(dr[k], ker[k], kv[k], vj[k], mj[k], sj[k]);
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) ent[k] = nxt[k];
     }
   } else {
-    scan(celli, pos_i, rebuild && keep);
+    QuadWriter out{nbb, (size_t)P.npb, i};
+    adami_scan<T>(P, S, c, celli, pos_i, contact, A, rebuild && keep ? &out : nullptr);
+    if (rebuild && keep) {
+      out.finish(list_entry(i, kOwnCell), IX_CAP);
+      S.nbb_cnt[lb][i] = out.cnt <= IX_CAP ? out.cnt : -1;
+    }
   }
   if (P.periodbound) {
     I3 cpb;
     V3<T> ppb;
-    if (period_image(P, celli, pos_i, true, cpb, ppb)) scan(cpb, ppb, false);
+    if (period_image(P, celli, pos_i, true, cpb, ppb)) adami_scan<T>(P, S, c, cpb, ppb, contact, A, nullptr);
   }
-  if (enorm(n_i) > T(0)) {
-    T nn = enorm(n_i);
-    S.cny[i] = V4<T>{n_i.x / nn, n_i.y / nn, n_i.z / nn, T(0)};
+  adami_finish(P, S, dyn, c, i, contact, code, pos_i, celli, A.n_i, A.rs, A.rps, A.rvr);
+}
+
+// The same with eight lanes per boundary particle (small cases, lists kept): the lanes form
+// the terms of eight list entries, then lanes 0..5 add the stress, the distance, the velocity,
+// the density with the kernel sum, and the normal.  Lists that overflowed are scanned by one
+// lane.  56k-particle wall (28k boundary): 31 -> 22 us a launch, column of 693: 15 -> 12.
+template <class T>
+__global__ void __launch_bounds__(kGroupThreads) k_adami_group(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
+  __shared__ GroupRows<T> sm;
+  const int lane = threadIdx.x & 31, l = lane & (kLanes - 1), g = lane / kLanes, warp = threadIdx.x >> 5;
+  const int row = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
+  const bool live = row < P.npb;
+  const int i = live ? row : P.npb - 1;
+  const int mode = dyn->ix_mode, lb = dyn->lbuf, c = dyn->cur_main;
+  if (live && l == 0 && mode == 0) S.dacc[lb][i] = 0.0f;  // candidate lists are rebuilt from these positions
+  if (dyn->npm == 0) return;
+  const V4<T>* __restrict__ pos = S.pos[c];
+  const V4<T>* __restrict__ vel = S.vel[c];
+  const V4<T>* __restrict__ idm = S.idm[c];
+  const V4<T>* __restrict__ sa = S.str_a[c];
+  const V2<T>* __restrict__ sb = S.str_b[c];
+  const unsigned* __restrict__ nbb = S.nbb[lb];
+  const V3<T> pos_i = ld3(pos, i);
+  const int4 cp = S.cellpos[c][i];
+  const I3 celli{cp.x, cp.y, cp.z};
+  const int4 code = S.codes[c][i];
+  const bool contact = code.x >= 10;
+  const T th = P.two_h;
+  const int cnt = live ? (dyn->list_ok ? S.nbb_cnt[lb][i] : -1) : 0;  // -1: no list, scanned
+  const unsigned own = list_entry(i, kOwnCell);
+  const int rounds = __reduce_max_sync(0xffffffffu, (max(cnt, 0) + kLanes - 1) / kLanes);
+  // rows: s.xx s.yy s.zz kv | s.xy s.xz s.yz ker m | distance (or normal, volume) | v | rho 1
+  const int y = l == 0 ? 0 : l == 1 ? 4 : l == 2 ? 8 : l == 3 ? 12 : l == 4 ? 16 : 8;
+  const int x = l == 2 ? 7 : l == 5 ? 11 : 3;
+  T acc[3] = {T(0), T(0), T(0)};
+  int e = l, buf = 0;
+  unsigned ent = group_entry(nbb, (size_t)P.npb, i, e, cnt, own);
+  for (int r = 0; r < rounds; ++r, e += kLanes, buf ^= 1) {
+    const int j = (int)(ent & kEntIdx);
+    const V4<T> pj = pos[j], vj = vel[j];
+    const T mj = idm[j].y;
+    const S6<T> sj = ld6(sa, sb, j);
+    const V3<T> off = mulI(entry_off(ent), th);
+    const bool valid = e < cnt, wall = j < P.npb;
+    ent = group_entry(nbb, (size_t)P.npb, i, e + kLanes, cnt, own);
+    V3<T> dr = pos_i - V3<T>{pj.x, pj.y, pj.z};
+    dr = dr - off;
+    const T r2 = pair_r2(dr.x, dr.y, dr.z);
+    const T q = pair_r(r2) * P.i_h;
+    const bool in = valid && r2 < P.r2_prefilter && q < T(2.0f);
+    const T ker = kernel_w(P.knorm, q);
+    const T kv = rmul(ker, mj / vj.w);
+    const V3<T> gk = dr * kernel_f(P.kgrad, q);
+    V4<T>* rows = sm.row[buf][warp][g];
+    V4<T>* mine = rows + l * (kRow / 4);
+    mine[0] = V4<T>{sj.xx, sj.yy, sj.zz, kv};
+    mine[1] = V4<T>{sj.xy, sj.xz, sj.yz, ker * mj};
+    mine[2] = wall ? V4<T>{gk.x, gk.y, gk.z, -P.vol_def} : V4<T>{dr.x, dr.y, dr.z, T(0)};
+    mine[3] = V4<T>{vj.x, vj.y, vj.z, T(0)};
+    mine[4] = V4<T>{vj.w, T(1), T(0), T(0)};
+    const unsigned mat = __ballot_sync(0xffffffffu, in && !wall), nrm = __ballot_sync(0xffffffffu, in && wall);
+    __syncwarp();
+    group_add(rows, x, y, (l == 5 ? nrm : mat) >> (g * kLanes) & 0xffu, acc);
   }
-  V4<T> vr_out = vel[i];
-  S6<T> str_out;
-  if (rps.w > T(0.0f)) {
-    const T kersum = rps.w;
-    const V3<T> dr_ref = xyz(rps);
-    const V4<T> nrm4 = S.normal[dyn->cur_nrm][i];
-    const T fcoef = nrm4.w;
-    const V3<T> nrm = xyz(nrm4);
-    const V3<T> vel_ref = xyz(rvr) / kersum;
-    const V3<T> vel_ref_n = nrm * dot(nrm, vel_ref);
-    const V3<T> vel_ref_t = vel_ref - vel_ref_n;
-    V3<T> vel_rb{T(0.0f), T(0.0f), T(0.0f)};
-    if (code.y == 1) {
-      const Motion<T>& mv = dyn->mv[code.w];
-      vel_rb = V3<T>{mv.trans_vel.x, mv.trans_vel.y, mv.trans_vel.z};
-      if (mv.is_rotat) {
-        V3<T> pabs = pos_i + mulI(celli, T(2.0f) * P.h);
-        V3<T> rp{mv.pos_rp.x, mv.pos_rp.y, mv.pos_rp.z};
-        V3<T> w{mv.rotat_vel.x, mv.rotat_vel.y, mv.rotat_vel.z};
-        vel_rb = vel_rb + cross(w, pabs - rp);
-      }
-    }
-    const V3<T> vel_rb_n = nrm * dot(nrm, vel_rb);
-    const V3<T> vel_rb_t = vel_rb - vel_rb_n;
-    const V3<T> vel_ext_n = vel_rb_n * T(2.0f) - vel_ref_n;
-    const V3<T> vel_ext_t = fcoef == T(-1.0f) ? vel_rb_t * T(2.0f) - vel_ref_t : vel_ref_t;
-    const V3<T> vel_ext = vel_ext_n + vel_ext_t;
-    const T rho = rvr.w / kersum;
-    vr_out = v4(vel_ext, rho);
-    if (contact) {
-      vr_out = v4(vel_rb, rho);
-      S.cvz[i] = V4<T>{vel_ext.x, vel_ext.y, vel_ext.z, T(0)};
-    }
-    const S6<T> str_ref = rs / kersum;
-    const V3<T> g{P.gravity[0], P.gravity[1], P.gravity[2]};
-    str_out = subdiag(str_ref, (g * dr_ref) / kersum);
-    S.vel[c][i] = vr_out;
-  } else {
-    str_out = zero6<T>();
+  const int b = g * kLanes;
+  const T a0 = acc[0], a1 = acc[1], a2 = acc[2];
+  S6<T> rs{from_lane(a0, b), from_lane(a1, b), from_lane(a2, b), from_lane(a0, b + 1), from_lane(a1, b + 1),
+           from_lane(a2, b + 1)};
+  V4<T> rps{from_lane(a0, b + 2), from_lane(a1, b + 2), from_lane(a2, b + 2), from_lane(a1, b + 4)};
+  V4<T> rvr{from_lane(a0, b + 3), from_lane(a1, b + 3), from_lane(a2, b + 3), from_lane(a0, b + 4)};
+  V3<T> n_i{from_lane(a0, b + 5), from_lane(a1, b + 5), from_lane(a2, b + 5)};
+  if (l != 0 || !live) return;
+  AdamiSums<T> sums{rs, rps, rvr, n_i};
+  if (cnt < 0) adami_scan<T>(P, S, c, celli, pos_i, contact, sums, nullptr);
+  if (P.periodbound) {
+    I3 cpb;
+    V3<T> ppb;
+    if (period_image(P, celli, pos_i, true, cpb, ppb)) adami_scan<T>(P, S, c, cpb, ppb, contact, sums, nullptr);
   }
-  st6(S.str_a[c], S.str_b[c], i, str_out);
-  write_rec(P, S.rec, i, S.pos[c][i], vr_out, str_out, P.vol_def * vr_out.w, contact);
+  adami_finish(P, S, dyn, c, i, contact, code, pos_i, celli, sums.n_i, sums.rs, sums.rps, sums.rvr);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1246,6 +1365,45 @@ template <bool Strict, class T> RWD void pair_eval(const Params<T>& P, const ISt
     }
   }
 }
+
+// The terms of pair_eval<false>, formed without a branch, whether or not the pair counts:
+// several pairs' chains (square root, division) then run side by side.
+template <class T> struct PairTerms {
+  V3<T> w, k, f, g;  // velocity difference, kernel gradient times volume, stress force, kernel gradient
+  T q, dvk, mass, visc, mv, tr;
+  bool wall;
+  RWD PairTerms(const Params<T>& P, const IState<T>& I, const V3<T> dr, const NbVals<T>& nb) {
+    using F = Fp<false>;
+    const T r2 = pair_r2(dr.x, dr.y, dr.z);
+    q = F::mul(r2 > T(0) ? r2 * f_rsqrt(r2) : T(0), P.i_h);
+    const T t = T(2.0f) - q;
+    const T dwdr = F::mul(F::mul(F::mul(P.kgrad, t), t), t);
+    g = V3<T>{F::mul(dr.x, dwdr), F::mul(dr.y, dwdr), F::mul(dr.z, dwdr)};
+    mass = nb.a.x;
+    wall = nb.a.y < T(0);
+    const T vol = f_abs(nb.a.y);
+    w = V3<T>{I.vel.x - nb.vr.x, I.vel.y - nb.vr.y, I.vel.z - nb.vr.z};
+    if (wall && I.shift == 1) w = V3<T>{T(0), T(0), T(0)};
+    k = V3<T>{F::mul(g.x, vol), F::mul(g.y, vol), F::mul(g.z, vol)};
+    dvk = F::dot3(w.x, w.y, w.z, k.x, k.y, k.z);
+    const S6<T> st{I.sor.xx + nb.a.z, I.sor.yy + nb.a.w, I.sor.zz + nb.b.x,
+                   I.sor.xy + nb.b.y, I.sor.xz + nb.b.z, I.sor.yz + nb.b.w};
+    f = V3<T>{F::dot3(st.xx, st.xy, st.xz, g.x, g.y, g.z), F::dot3(st.xy, st.yy, st.yz, g.x, g.y, g.z),
+              F::dot3(st.xz, st.yz, st.zz, g.x, g.y, g.z)};
+    visc = F::dot3(w.x, w.y, w.z, dr.x, dr.y, dr.z);
+    mv = F::mul(mass, f_fastdiv(F::mul(P.visc_k, visc), F::mul(r2 + P.eta, F::mul(T(0.5f), I.rho + nb.vr.w))));
+    tr = nb.a.z + nb.a.w + nb.b.x;
+  }
+  // mass times the artificial stress, 0 without one
+  RWD T artificial(const Params<T>& P, const IState<T>& I) const {
+    using F = Fp<false>;
+    if (P.art_coef == T(0.f)) return T(0);
+    const T rj = tr > T(0.0f) ? F::mul(tr, P.art_coef) : T(0.0f);
+    const T artp = I.ri + rj;
+    if (!(artp > T(0.0f))) return T(0);
+    return F::mul(mass, F::mul(artp, f_pow(kernel_w(P.knorm, q) / P.kernel_dr, P.kernel_zero / P.kernel_dr)));
+  }
+};
 
 template <bool Strict, class T> RWD void pair_term(const Params<T>& P, const IState<T>& I, const V3<T> dr,
                                                    const Rec<T>* __restrict__ rec, int j, Acc<T>& A) {
@@ -1763,7 +1921,8 @@ template <bool Strict, class T> RWD void ix_finish(const Params<T>& P, const Dev
 // then evaluates the lists with the same pairs in the same order as a scan.  One thread
 // per particle, boundary rows first, so that in an update the Adami kernel (many
 // registers, few warps per SM) only walks lists.
-template <class T> __global__ void __launch_bounds__(256) k_build_lists(const Params<T> P, DevState<T> S, Dyn<T>* dyn) {
+template <class T>
+__global__ void __launch_bounds__(256) k_build_lists(const Params<T> P, DevState<T> S, Dyn<T>* dyn, int bnd) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   const int mode = dyn->ix_mode;
   if (!S.nbg[0] || !P.keep_lists || mode == 1) return;
@@ -1784,6 +1943,7 @@ template <class T> __global__ void __launch_bounds__(256) k_build_lists(const Pa
     S.queue[base + __popc(m & ((1u << lane) - 1u))] = row;
   };
   if (row < P.npb) {
+    if (mode == 0 && bnd) enqueue();
     if (mode == 2 && S.nbb[0]) {
       const int4 cb = S.cellpos[c][row];
       if (near_marked(P, S, dyn, I3{cb.x, cb.y, cb.z})) enqueue();
@@ -1841,7 +2001,8 @@ template <class T> __global__ void __launch_bounds__(256) k_build_lists(const Pa
 }
 
 // The lists queued by a list update (soil rows' interaction lists and boundary rows'
-// Adami lists), one warp per list: the 27 cells x 2 ranges are 54 segments of
+// Adami lists; in a full build with eight lanes per particle, every boundary row's), one
+// warp per list: the 27 cells x 2 ranges are 54 segments of
 // candidates, flattened in the scan's order; the warp tests 32 consecutive candidates
 // at a time and appends the hits in order (ballot + prefix count), so the list holds
 // the pairs a full build lists, in the same order.  The displacement bounds run on.
@@ -1849,9 +2010,9 @@ template <class T> __global__ void __launch_bounds__(256) k_rebuild_lists(const 
   constexpr int kSeg = 54, kWarps = 256 / 32;
   __shared__ int seg_beg[kWarps][kSeg + 1];  // first flattened candidate of each segment
   __shared__ int seg_j0[kWarps][kSeg];       // first particle index of each segment
-  if (!S.nbg[0] || !P.keep_lists || dyn->ix_mode != 2) return;
+  if (!S.nbg[0] || !P.keep_lists || dyn->ix_mode == 1) return;
   const int nq = dyn->n_queue;
-  if (blockIdx.x == 0 && threadIdx.x == 0) dyn->n_rebuilt += nq;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && dyn->ix_mode == 2) dyn->n_rebuilt += nq;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lb = dyn->lbuf, c = dyn->cur_main;
   const V4<T>* __restrict__ pos = S.pos[c];
@@ -1987,6 +2148,81 @@ __global__ void __launch_bounds__(Walk ? IX_WALK_MAX_THREADS : IX_THREADS, Walk 
   else ix_sums_global<Strict>(P, S, c, celli, I, nbl + threadIdx.x, blockDim.x, IX_CAP, A);
   if (P.periodbound) ix_period<Strict>(P, S, c, i, celli, I, A);
   ix_finish<Strict>(P, S, c, cpar, i, celli, I, A, cv);
+}
+
+// The walk with eight lanes per particle (see GroupRows), for cases that a thread per particle
+// leaves waiting.  The terms are pair_eval<false>'s; lanes 0..2 add the rows of the velocity
+// gradient, 3 the stress force, 4 the viscous one, 5 the artificial stress, 6 the density rate.
+// 693-particle column 15 us a launch against 28, 5.4k in FP64 32 against 54.  What bounds it
+// when it fills the GPU is the L1 data stage (73% of its wavefronts at 28k): per eight
+// entries the rows cost as many again as the record gathers, so beyond some 16k particles
+// the thread per particle is faster (41 us against 36 at 28k).
+template <class T>
+__global__ void __launch_bounds__(kGroupThreads) k_interaction_group(const Params<T> P, DevState<T> S, const Dyn<T>* dyn,
+                                                                     int cpar) {
+  __shared__ GroupRows<T> sm;
+  const int lane = threadIdx.x & 31, l = lane & (kLanes - 1), g = lane / kLanes, warp = threadIdx.x >> 5;
+  const int t0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
+  const int npm = dyn->npm, lb = dyn->lbuf, c = dyn->cur_main;
+  if (npm == 0) return;
+  const int t = min(t0, npm - 1), i = P.npb + t;
+  const int kept = t0 < npm ? S.nbg_cnt[lb][t] : -1;  // -1: the scan launch takes this particle
+  const int cnt = max(kept, 0);
+  const int rounds = __reduce_max_sync(0xffffffffu, (cnt + kLanes - 1) / kLanes);
+  const V4<T> cv = S.cv[cpar][i];
+  IState<T> I;
+  Acc<T> A;
+  ix_begin<false>(P, S, c, i, cv, I, A);
+  const Rec<T>* __restrict__ rec = S.rec;
+  const unsigned* __restrict__ lists = S.nbg[lb];
+  const size_t stride = (size_t)S.nbg_stride;
+  const unsigned own = list_entry(i, kOwnCell);
+  const T th = P.two_h;
+  // rows: k.x k.y k.z -w.x | f.x f.y f.z -w.y | g.x g.y g.z -w.z | dvk 0 0 mass | mv -ma rho_i 0
+  const int y = l < 3 ? 0 : l == 3 ? 4 : l < 6 ? 8 : 12;
+  const int x = l < 3 ? 3 + 4 * l : l == 3 ? 15 : l < 6 ? 12 + l : 18;
+  T acc[3] = {T(0), T(0), T(0)};
+  int e = l, buf = 0;
+  unsigned ent = group_entry(lists, stride, t, e, cnt, own), nxt = group_entry(lists, stride, t, e + kLanes, cnt, own);
+  NbVals<T> nb = load_nb(rec, (int)(ent & kEntIdx));
+  for (int r = 0; r < rounds; ++r, e += kLanes, buf ^= 1) {
+    const NbVals<T> cur = nb;
+    const I3 off = entry_off(ent);
+    ent = nxt;
+    nb = load_nb(rec, (int)(ent & kEntIdx));
+    nxt = group_entry(lists, stride, t, e + 2 * kLanes, cnt, own);
+    const V3<T> dr{f_fma((T)-off.x, th, I.pos.x - cur.p.x), f_fma((T)-off.y, th, I.pos.y - cur.p.y),
+                   f_fma((T)-off.z, th, I.pos.z - cur.p.z)};
+    const PairTerms<T> p(P, I, dr, cur);
+    const bool in = e < cnt && p.q < T(2.0f), wall = p.wall;
+    const T ma = in && !wall ? p.artificial(P, I) : T(0);
+    V4<T>* rows = sm.row[buf][warp][g];
+    V4<T>* mine = rows + l * (kRow / 4);
+    mine[0] = V4<T>{p.k.x, p.k.y, p.k.z, -p.w.x};
+    mine[1] = V4<T>{p.f.x, p.f.y, p.f.z, -p.w.y};
+    mine[2] = V4<T>{p.g.x, p.g.y, p.g.z, -p.w.z};
+    mine[3] = V4<T>{p.dvk, T(0), T(0), p.mass};
+    mine[4] = V4<T>{p.mv, -ma, I.rho, T(0)};
+    const unsigned b_in = __ballot_sync(0xffffffffu, in), b_mat = __ballot_sync(0xffffffffu, in && !wall);
+    const unsigned b_visc = __ballot_sync(0xffffffffu, in && !wall && p.visc < T(0.0f) && P.viscosity_type == 1);
+    const unsigned b_art = __ballot_sync(0xffffffffu, ma != T(0));
+    const unsigned on = l < 3 ? b_in : l == 4 ? b_visc : l == 5 ? b_art : b_mat;
+    __syncwarp();
+    group_add(rows, x, y, on >> (g * kLanes) & 0xffu, acc);
+  }
+  const int b = g * kLanes;
+  const T a0 = acc[0], a1 = acc[1], a2 = acc[2];
+  A.gv = F9<T>{from_lane(a0, b), from_lane(a1, b), from_lane(a2, b), from_lane(a0, b + 1), from_lane(a1, b + 1),
+               from_lane(a2, b + 1), from_lane(a0, b + 2), from_lane(a1, b + 2), from_lane(a2, b + 2)};
+  A.s = V3<T>{from_lane(a0, b + 3), from_lane(a1, b + 3), from_lane(a2, b + 3)};
+  A.av = V3<T>{from_lane(a0, b + 4), from_lane(a1, b + 4), from_lane(a2, b + 4)};
+  A.as = V3<T>{from_lane(a0, b + 5), from_lane(a1, b + 5), from_lane(a2, b + 5)};
+  A.accden = from_lane(a0, b + 6);
+  if (l != 0 || kept < 0) return;
+  const int4 cp = S.cellpos[c][i];
+  const I3 celli{cp.x, cp.y, cp.z};
+  if (P.periodbound) ix_period<false>(P, S, c, i, celli, I, A);
+  ix_finish<false>(P, S, c, cpar, i, celli, I, A, cv);
 }
 
 // ---------------------------------------------------------------------------------
@@ -2258,6 +2494,8 @@ template <class T, bool Strict> __global__ void __launch_bounds__(IX2_TB) k_inte
 // 100 spilled bytes): they stream about 300 B per particle, and at the two blocks
 // their natural 94 registers allow they wait on memory (measured 19% faster at
 // three blocks, another 5% at four).
+// In FP64 four blocks spill 500 to 800 bytes; two (128 registers) take 18 us instead of 26 at
+// 60k particles and 28 instead of 31 to 33 at 112k (three: 23 and 28, one: 23 and 34).
 // One row of the predictor.  With the learned closure on, HypoCS rows keep their stress
 // here and the closure's pass updates it (and writes their record).
 template <class T> RWD void predictor_row(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i) {
@@ -2321,7 +2559,7 @@ template <class T> RWD void predictor_row(const Params<T>& P, const DevState<T>&
 }
 
 template <class T>
-__global__ void __launch_bounds__(256, 4) k_predictor(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_predictor(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
   predictor_row(P, S, dyn, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -2477,7 +2715,7 @@ template <class T> RWD void corrector_row(const Params<T>& P, const DevState<T>&
 }
 
 template <class T>
-__global__ void __launch_bounds__(256, 4) k_corrector(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_corrector(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
   corrector_row(P, S, dyn, blockIdx.x * blockDim.x + threadIdx.x);
 }
 

@@ -1,10 +1,12 @@
-"""The packed walk of the interaction (two list entries at a time, predicated sums) against
-the chunked kernel, which evaluates every pair by itself with scalar instructions: every sum
-is the same, so the states agree bit for bit."""
+"""The walks of the interaction against the chunked kernel, which evaluates every pair by
+itself: eight lanes per particle (a small case alone), and the packed walk of one thread per
+particle (the same case beside a large one in a batch: two list entries at a time, predicated
+sums).  Every sum is the same, so the states agree bit for bit."""
 import numpy as np
 import pytest
 
 from retainwall_code_b200 import LoquatSph, _abi, cases as C
+from retainwall_code_b200.sph import Batch
 
 pytestmark = pytest.mark.gpu
 
@@ -61,15 +63,66 @@ CASES = {
 }
 
 
+def _step(sim, steps, beside):
+    if not beside:
+        sim.step(steps)
+        return
+    big = LoquatSph(case=C.retaining_wall(nx=40, ny=25, nz=20, seed=1), precision=sim.precision)
+    batch = Batch([sim, big])
+    batch.step(steps)
+    batch.synchronize()
+    batch.close()
+
+
+@pytest.mark.parametrize("beside", [False, True])
 @pytest.mark.parametrize("skin", [0.02, 0.4])
 @pytest.mark.parametrize("name", CASES)
-def test_packed_walk_equals_single_pairs(name, skin):
+def test_packed_walk_equals_single_pairs(name, skin, beside):
     make, steps = CASES[name]
     a, b = LoquatSph(case=make()), LoquatSph(case=make())
     a.set_option(_abi.OPT_LIST_SKIN, skin)
     b.set_option(_abi.OPT_INTERACTION_KERNEL, 1)
-    a.step(steps)
+    _step(a, steps, beside)
     b.step(steps)
     for key in KEYS:
         np.testing.assert_array_equal(a.get(key), b.get(key), err_msg=key)
     assert a.list_stats()[1] == a.info().npm  # every particle walked a list
+
+
+@pytest.mark.parametrize("beside", [False, True])
+def test_walks_in_fp64(beside):
+    """FP64 through cell changes (lists rebuilt, carried and updated), against the scan."""
+    c = C.column_collapse(11, 9, 13, seed=11)
+    c.velrhop[c.npb:, 0] = 0.5
+    a, b = LoquatSph(case=c, precision=8), LoquatSph(case=c, precision=8)
+    b.set_option(_abi.OPT_LIST_SKIN, 0.0)
+    _step(a, 60, beside)
+    b.step(60)
+    for key in KEYS:
+        np.testing.assert_array_equal(a.get(key), b.get(key), err_msg=key)
+    assert a.info().n_list_updates > 0
+
+
+@pytest.mark.parametrize("when", ["search", "write"])
+def test_lists_dropped_between_stages(when):
+    """Stage calls with the interaction kernel changed, or an array written, between the
+    search and the boundary stage: no stale list is walked."""
+    c = C.retaining_wall(nx=9, ny=6, nz=7, mode="passive", wall_speed=0.02, seed=3)
+    a, b = LoquatSph(case=c), LoquatSph(case=c)
+    a.step(3)
+    b.step(3)
+    for s in (a, b):
+        s.set_option(_abi.OPT_LIST_SKIN, 0.0 if s is b else 0.02)
+        if when == "search":
+            s.set_option(_abi.OPT_INTERACTION_KERNEL, 1)
+        s.step_calculation()
+        s.neighbor_search(0)
+        if when == "search":
+            s.set_option(_abi.OPT_INTERACTION_KERNEL, 0)
+        else:
+            s.set("velrhop", s.get("velrhop"))
+        s.rigid_body_update()
+        s.adami_boundary()
+        s.find_corner_particle()
+    for key in KEYS:
+        np.testing.assert_array_equal(a.get(key), b.get(key), err_msg=key)
