@@ -111,6 +111,7 @@ template <class T> struct Engine final : EngineBase {
   double* d_clstats = nullptr;
   unsigned long long* d_count = nullptr;
   int nsm = 148;
+  SortPlan sort{};
   size_t near_wall_words = 0;
   // Step graphs captured with conditional nodes (gated()); st_body captures their bodies.
   bool allow_cond = false;
@@ -351,12 +352,12 @@ template <class T> struct Engine final : EngineBase {
       S.tk = dalloc<int>(np);
       S.tv = dalloc<int>(np);
       S.range = dalloc<int2>(P.ncell);
-      S.ntiles = (int)nblk((long)np, RS_TILE);
-      S.hist = dalloc<int>(256 * (size_t)S.ntiles);
-      S.dtot = dalloc<int>(256);
       int bits = 1;
       while ((1L << bits) <= P.ncell_delete_m) ++bits;
-      S.sort_passes = (bits + 7) / 8;
+      sort = sort_plan((long)np, bits, SIZE_MAX);
+      S.hist = dalloc<int>(sort.hist());
+      S.dtot = dalloc<int>(sort.bins());
+      S.sort_passes = sort.passes;
       S.skeys = (S.sort_passes & 1) ? S.tk : S.keys;
       S.sperm = (S.sort_passes & 1) ? S.tv : S.vals;
       S.wsum = dalloc<double>(3 * (WF_BLOCKS + 1));
@@ -497,6 +498,9 @@ template <class T> struct Engine final : EngineBase {
                                (int)sizeof(Ix2Smem<T>)));
     RW_CU(cudaFuncSetAttribute(k_interaction2<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(Ix2Smem<T>)));
+    for (auto* f : {k_rs_downsweep<4>, k_rs_downsweep<8>, k_rs_downsweep<16>})
+      RW_CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)rs_down_smem(1 << RS_MAX_BITS, 16 * RS_THREADS)));
     search(0);  // the first cell sort; the lists are built with the first step's boundary stage
     RW_CU(cudaStreamSynchronize(st));
   }
@@ -557,10 +561,7 @@ template <class T> struct Engine final : EngineBase {
               const int* vi = (pass & 1) ? S.tv : S.vals;
               int* ko = (pass & 1) ? S.keys : S.tk;
               int* vo = (pass & 1) ? S.vals : S.tv;
-              k_rs_upsweep<<<S.ntiles, RS_THREADS, 0, st>>>(ki, np, 8 * pass, S.hist, S.ntiles, need_ptr());
-              k_rs_scan<<<256, RS_THREADS, 0, st>>>(S.hist, S.ntiles, S.dtot, need_ptr());
-              k_rs_downsweep<<<S.ntiles, RS_THREADS, 0, st>>>(ki, vi, ko, vo, np, 8 * pass, S.hist, S.dtot, S.ntiles,
-                                                              need_ptr());
+              rs_pass(sort, ki, vi, ko, vo, np, pass, S.hist, S.dtot, need_ptr(), st);
             }
             k_clear_if<<<2 * nsm, 256, 0, st>>>(reinterpret_cast<unsigned*>(S.range), 2 * (size_t)P.ncell, dirty);
             k_ranges<T><<<nblk(np, 256), 256, 0, st>>>(P, S, d_dyn);

@@ -16,16 +16,16 @@
 namespace {
 
 constexpr int kMaxKeys = RW_NOALLOC_MAX_KEYS;
-constexpr int kMaxTiles = (kMaxKeys + rw::RS_TILE - 1) / rw::RS_TILE;
+constexpr int kMaxCounts = 256 * 512, kMaxBins = 256;
 
 // Scratch: ping-pong keys/values, per-tile digit counts, digit totals, sort flag:
 // 2 x 2^20 + 256 x 512 + 257 ints = 8,913,924 bytes (8.9 MB, 8.5 MiB).
 struct Scratch {
   int tk[kMaxKeys];
   int tv[kMaxKeys];
-  int hist[256 * kMaxTiles];
-  int dtot[256];
-  int need;
+  int hist[kMaxCounts];
+  int dtot[kMaxBins];
+  int spare;  // keeps the stated size
 };
 static __device__ __align__(256) Scratch g_scratch;
 
@@ -48,13 +48,6 @@ int scratch_for_current_device(Scratch** out) {
   return RW_OK;
 }
 
-__global__ void k_fill_iota(int* v, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = i;
-}
-
-__global__ void k_set_flag(int* f) { *f = 1; }
-
 }  // namespace
 
 extern "C" rw_status rw_cell_sort_noalloc(const int32_t* d_keys, int32_t n, int32_t max_key, int32_t* d_sorted_keys,
@@ -68,29 +61,20 @@ extern "C" rw_status rw_cell_sort_noalloc(const int32_t* d_keys, int32_t n, int3
   cudaStream_t st = (cudaStream_t)stream;
   int bits = 1;
   while ((1 << bits) <= max_key) ++bits;
-  const int passes = (bits + 7) / 8;
-  const int ntiles = (n + rw::RS_TILE - 1) / rw::RS_TILE;
-  // The permutation starts as the identity in the output buffer; the sort flag is
-  // set because every call sorts (the array keeps the previous call's contents).
-  k_fill_iota<<<(n + 255) / 256, 256, 0, st>>>(d_perm, n);
-  k_set_flag<<<1, 1, 0, st>>>(&s->need);
+  // eight-bit digits: the scratch holds 256 totals (and whole bytes of the keys are compared,
+  // whatever max_key)
+  const rw::SortPlan plan = rw::sort_plan(n, (bits + 7) / 8 * 8, kMaxCounts, 8);
+  const int passes = plan.passes;
   // Ping-pong between (sorted_keys, perm) and the scratch pair, arranged so the last
-  // pass writes the caller's outputs; the first pass reads the caller's keys.
+  // pass writes the caller's outputs; the first pass reads the caller's keys and numbers
+  // them itself (no values yet).
   const int* kin = d_keys;
-  const int* vin = d_perm;
+  const int* vin = nullptr;
   for (int p = 0; p < passes; ++p) {
     const bool to_out = ((passes - 1 - p) % 2) == 0;
     int* ko = to_out ? d_sorted_keys : s->tk;
     int* vo = to_out ? d_perm : s->tv;
-    if (p == 0 && to_out) {  // odd pass count (1 or 3): pass 0 writes the caller's outputs, so
-                             // its values come from an identity in the scratch (not in place)
-      k_fill_iota<<<(n + 255) / 256, 256, 0, st>>>(s->tv, n);
-      vin = s->tv;
-    }
-    rw::k_rs_upsweep<<<ntiles, rw::RS_THREADS, 0, st>>>(kin, n, 8 * p, s->hist, ntiles, &s->need);
-    rw::k_rs_scan<<<256, rw::RS_THREADS, 0, st>>>(s->hist, ntiles, s->dtot, &s->need);
-    rw::k_rs_downsweep<<<ntiles, rw::RS_THREADS, 0, st>>>(kin, vin, ko, vo, n, 8 * p, s->hist, s->dtot, ntiles,
-                                                         &s->need);
+    rw::rs_pass(plan, kin, vin, ko, vo, n, p, s->hist, s->dtot, nullptr, st);
     kin = ko;
     vin = vo;
   }
