@@ -96,6 +96,9 @@ template <class T> struct Engine final : EngineBase {
   int cpar = 0;  // live contact buffer
   bool compat_contact = true;
   cudaGraphExec_t gexec = nullptr;
+  cudaGraphExec_t gsearch[2] = {nullptr, nullptr};  // neighbor_search of a stage call, by section
+  bool gsearch_refused = false;
+  int stage_searches = 0;
   int g_cpar = -1;
   int ix_kernel = 0;     // 0: neighbours through L1/L2 (default); 1: chunked, shared-memory position tile
   int walk_threads = 128;   // RW_OPT_WALK_THREADS: block size of the walk launch
@@ -130,7 +133,7 @@ template <class T> struct Engine final : EngineBase {
   ~Engine() override {
     wait_save();
     if (stage_h) cudaFreeHost(stage_h);
-    if (gexec) cudaGraphExecDestroy(gexec);
+    drop_graphs();
     if (st) cudaStreamSynchronize(st);
     for (void* p : allocs) cudaFree(p);
     if (st) cudaStreamDestroy(st);
@@ -519,6 +522,52 @@ template <class T> struct Engine final : EngineBase {
   // The search, then the candidate lists, built or updated (only when they do not
   // stand), before the boundary and corner stages so that the corner search walks them.
   void neighbor_search(int section) override {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    RW_CU(cudaStreamIsCapturing(st, &cs));
+    if (cs == cudaStreamCaptureStatusNone && graph_gates && ++stage_searches > 4 && search_graph(section)) {
+      RW_CU(cudaGraphLaunch(gsearch[section], st));
+      return;
+    }
+    launch_search(section);
+  }
+  // The search of a stage call as a graph of its own, behind the same gates as in the step
+  // graph: most searches have nothing to do, and their 17 launches that return at once cost
+  // more than a small case's kernels (56k-particle wall, stage calls: 0.37 ms a step, 0.27
+  // this way).  Made once a host program has called the stages for two steps (0.15 ms each).
+  // False: conditional nodes refused, launched plainly.
+  bool search_graph(int section) {
+    if (gsearch[section]) return true;
+    if (gsearch_refused) return false;
+    cudaGraph_t g = nullptr;
+    RW_CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    allow_cond = true;
+    cudaError_t e = cudaSuccess;
+    try {
+      launch_search(section);
+    } catch (const Fail&) {
+      e = cudaErrorNotSupported;
+    }
+    allow_cond = false;
+    const cudaError_t ended = cudaStreamEndCapture(st, &g);
+    if (e == cudaSuccess) e = ended;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&gsearch[section], g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      gsearch[section] = nullptr;
+      gsearch_refused = true;
+    }
+    return e == cudaSuccess;
+  }
+  // Captured launches hold the parameters and options of their capture.
+  void drop_graphs() {
+    for (cudaGraphExec_t* g : {&gexec, &gsearch[0], &gsearch[1]})
+      if (*g) {
+        cudaGraphExecDestroy(*g);
+        *g = nullptr;
+      }
+  }
+  void launch_search(int section) {
     search(section);
     if (lists_kept()) {
       gated([&](cudaGraphConditionalHandle h) { k_build_gate<T><<<1, 1, 0, st>>>(P, S, d_dyn, h); },
@@ -670,10 +719,7 @@ template <class T> struct Engine final : EngineBase {
   // Learned closure.
   // ------------------------------------------------------------------------------
   int set_closure(rw_mlp* net, double margin) override {
-    if (gexec) {  // the closure launches are part of the captured step
-      cudaGraphExecDestroy(gexec);
-      gexec = nullptr;
-    }
+    drop_graphs();  // the closure launches are part of the captured step
     ++generation;
     if (!net) {
       P.closure = 0;
@@ -1072,10 +1118,7 @@ template <class T> struct Engine final : EngineBase {
     } else {
       return RW_EINVAL;
     }
-    if (gexec) {  // parameters are baked into the captured graph
-      cudaGraphExecDestroy(gexec);
-      gexec = nullptr;
-    }
+    drop_graphs();  // parameters are baked into the captured graphs
     ++generation;
     return RW_OK;
   }

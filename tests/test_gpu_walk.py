@@ -126,3 +126,28 @@ def test_lists_dropped_between_stages(when):
         s.find_corner_particle()
     for key in KEYS:
         np.testing.assert_array_equal(a.get(key), b.get(key), err_msg=key)
+
+
+def test_stage_calls_equal_steps_across_an_option():
+    """Stage calls whose searches run as captured graphs (from the third step on), through
+    cell changes and an option that drops the captures, against whole steps."""
+    c = C.column_collapse(8, 7, 9, seed=12)
+    c.velrhop[c.npb:, 0] = 0.5
+    a, b = LoquatSph(case=c), LoquatSph(case=c)
+
+    def stages(n):
+        for _ in range(n):
+            a.step_calculation()
+            a.predictor_section()
+            a.corrector_section()
+            a.end_step()
+
+    stages(12)
+    b.step(12)
+    for s in (a, b):
+        s.set_option(_abi.OPT_LIST_SKIN, 0.3)
+    stages(12)
+    b.step(12)
+    for key in KEYS + ["cellpos", "codes"]:
+        np.testing.assert_array_equal(a.get(key), b.get(key), err_msg=key)
+    assert a.info().n_sorts > 3 and a.info().device_err == 0
