@@ -132,7 +132,7 @@ def test_stage_calls_equal_steps_across_an_option():
     """Stage calls whose searches run as captured graphs (from the third step on), through
     cell changes and an option that drops the captures, against whole steps."""
     c = C.column_collapse(8, 7, 9, seed=12)
-    c.velrhop[c.npb:, 0] = 0.5
+    c.velrhop[c.npb:, 0] = 5.0  # about 0.03 dx a step: the first cell changes after two steps
     a, b = LoquatSph(case=c), LoquatSph(case=c)
 
     def stages(n):
