@@ -6,11 +6,9 @@
 // Training step (one launch per minibatch, one 128-sample tile per loop iteration):
 //   forward  : five tcgen05 MMAs per tile (BF16 operands in shared memory, FP32 in
 //              TMEM); the four hidden pre-activations stay in TMEM for the backward pass;
-//   backward : dH(l-1) = G(l) W(l) on tcgen05 (G in BF16, as it feeds the MMA);
-//              dW(l) = H(l-1)^T G(l) and db(l) = sum G(l) on the CUDA cores in FP32,
-//              accumulated per block in shared memory (there is no TMEM or shared memory
-//              left for a third set of transposed operand tiles), then added to the
-//              global gradient once per launch;
+//   backward : dH(l-1) = G(l) W(l) and dW(l) = H(l-1)^T G(l) on tcgen05 (G in BF16, as it
+//              feeds the MMAs), db(l) = sum G(l) on the CUDA cores in FP32, all accumulated
+//              per block in shared memory, then added to the global gradient once per launch;
 //   update   : Adam on the FP32 master parameters, which also re-packs the BF16
 //              operand tiles.
 #include <cuda_runtime.h>
@@ -71,19 +69,21 @@ __global__ void k_pack(const float* __restrict__ p, unsigned char* fw, unsigned 
 
 // Adam step on every parameter (bias-corrected), re-packing the operands; clears the
 // gradient for the next minibatch.
+__device__ __forceinline__ int acc_index(int k);
 __global__ void k_adam(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                        float lr, float b1, float b2, float eps, float bc1, float bc2, unsigned char* fw,
                        unsigned char* bw, float* bias) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= NPARAM) return;
-  const float gk = g[k];
+  const int a = acc_index(k);  // the gradient lies as the training kernel accumulates it
+  const float gk = g[a];
   const float mk = b1 * m[k] + (1.0f - b1) * gk;
   const float vk = b2 * v[k] + (1.0f - b2) * gk * gk;
   m[k] = mk;
   v[k] = vk;
   const float w = p[k] - lr * (mk / bc1) / (sqrtf(vk / bc2) + eps);
   p[k] = w;
-  g[k] = 0.0f;
+  g[a] = 0.0f;
   pack_param(k, w, fw, bw, bias);
 }
 
@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(TILE) k_forward(Net net, const float* __restri
 // ---------------------------------------------------------------------------------
 // Training: forward + backward of a minibatch, gradient accumulated into grad.
 // ---------------------------------------------------------------------------------
+constexpr int TRAIN_THREADS = 2 * TILE, BPARTS = TRAIN_THREADS / HID;
 struct TrainSmem {
   alignas(128) unsigned char fw[FWBYTES];
   alignas(128) unsigned char bw[BWBYTES];
@@ -131,9 +132,10 @@ struct TrainSmem {
   alignas(128) unsigned char h[NHID][TILE * HID * 2];
   alignas(128) unsigned char g[TILE * HID * 2];
   alignas(128) unsigned char g5[TILE * OUTP * 2];
+  alignas(16) float bias[NBIAS];
   float acc[NPARAM];
-  float bias[NBIAS];
-  uint64_t bar;
+  float bacc[BPARTS][NBIAS];  // bias gradients, by part of the tile's rows
+  uint64_t bar, wbar;         // MMAs; weight copies
   uint32_t tmem;
   int err;
 };
@@ -155,37 +157,36 @@ __device__ __forceinline__ void issue_wgrad(const unsigned char* a_tile, int Ka,
                  idesc, ks > 0 ? 1u : 0u);
 }
 
-// Adds a 64 x N accumulator (M = 64 layout: row r in TMEM lane 32 (r / 16) + r % 16, so
-// lanes 0..15 of warp w hold rows 16 w .. 16 w + 15) into acc[base + col * 64 + row], for
-// the columns col < ncols.  tcol: the accumulator's first column.  Every lane takes part
-// in the TMEM loads; lanes 16..31 discard theirs.
+// Adds columns [c0, c0 + N) of a 64-row accumulator (M = 64 layout: row r in TMEM lane
+// 32 (r / 16) + r % 16, so lanes 0..15 of warps w and w + 4 hold rows 16 (w % 4) .. + 15) into
+// acc[base + col * 64 + row], for the columns below ncols.  tcol: the accumulator's first
+// column.  Every lane takes part in the TMEM load; lanes 16..31 discard theirs.
 template <int N>
-__device__ __forceinline__ void add_wgrad(float* acc, uint32_t tmem, uint32_t tcol, int base, int ncols) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const uint32_t taddr = tmem + ((uint32_t)(w * 32) << 16) + tcol;
+__device__ __forceinline__ void add_wgrad(float* acc, uint32_t tmem, uint32_t tcol, int c0, int base, int ncols) {
+  const int w = (threadIdx.x >> 5) & 3, l = threadIdx.x & 31;
+  const uint32_t taddr = tmem + ((uint32_t)(w * 32) << 16) + tcol + (uint32_t)c0;
   const int r = 16 * w + l;
+  float v[N];
+  if constexpr (N == 32) tc::tmem_ld32(taddr, v);
+  else tc::tmem_ld16(taddr, v);
+  if (l < 16)
 #pragma unroll
-  for (int c = 0; c < N; c += 16) {
-    float v[16];
-    tc::tmem_ld16(taddr + (uint32_t)c, v);
-    if (l < 16)
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        if (c + k < ncols) acc[base + (c + k) * 64 + r] += v[k];
-  }
+    for (int k = 0; k < N; ++k)
+      if (c0 + k < ncols) acc[base + (c0 + k) * 64 + r] += v[k];
 }
 
-// acc[b0 + o] += sum over the tile's 128 rows of G[b][o], for o < NB (G: 128 x Kg tile).
-// Thread o sums column o; the rows are visited in an order rotated by o / 8, so the four
-// 8-column groups of a warp read different banks.
+// bacc[part][o] += sum over the part's rows of G[b][o], for o < NB (G: 128 x Kg tile); the
+// parts are 128 / BPARTS rows each, one thread per part and column.  The rows are visited in
+// an order rotated by o / 8, so the four 8-column groups of a warp read different banks.
 template <int Kg, int NB>
-__device__ __forceinline__ void add_bias_grad(float* acc, int b0, const unsigned char* g) {
-  const int o = threadIdx.x;
+__device__ __forceinline__ void add_bias_grad(float (*bacc)[NBIAS], int b0, const unsigned char* g) {
+  constexpr int kRows = TILE / BPARTS;
+  const int o = threadIdx.x % HID, part = threadIdx.x / HID;
   if (o >= NB) return;
   float t = 0.0f;
 #pragma unroll 8
-  for (int k = 0; k < TILE; ++k) t += load_elem<Kg>(g, (k + (o >> 3)) & (TILE - 1), o);
-  acc[b0 + o] += t;
+  for (int k = 0; k < kRows; ++k) t += load_elem<Kg>(g, part * kRows + ((k + (o >> 3)) & (kRows - 1)), o);
+  bacc[part][b0 + o] += t;
 }
 
 // The accumulator layout of the weight gradients in shared memory: W1 as the parameters
@@ -203,27 +204,41 @@ __device__ __forceinline__ int acc_index(int k) {
   return k;
 }
 
-__global__ void __launch_bounds__(TILE, 1) k_train(Net net, const float* __restrict__ X, const float* __restrict__ Tg,
-                                                long long n_all, long long first, int n, long long sa, long long sc,
-                                                float inv_count, float* __restrict__ grad, double* __restrict__ loss,
-                                                int* err) {
+// Gradient in parameter order (the training kernel leaves it as it accumulates it).
+__global__ void k_grad_order(const float* __restrict__ g, float* __restrict__ out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < NPARAM) out[k] = g[acc_index(k)];
+}
+
+// One block per 128-sample tile at a time, two warps per 32 rows (each half of the columns).
+// What bounds a launch is one tile's chain: ten layers of MMA, TMEM load, 8192 tanh on 16
+// lanes a cycle (0.26 us a layer) and the barriers between them; a minibatch of 8192 is 64
+// tiles on 148 SMs.  So the rows are split over two warps, the bias sums over four parts,
+// the weights come by bulk copies while the samples are gathered, and the accumulators leave
+// in the order they lie in (in parameter order every lane of a warp read the same bank):
+// 50 us a minibatch of 8192 with its update before, 24 now.
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(Net net, const float* __restrict__ X,
+                                                         const float* __restrict__ Tg, long long n_all, long long first,
+                                                         int n, long long sa, long long sc, float inv_count,
+                                                         float* __restrict__ grad, double* __restrict__ loss, int* err) {
   extern __shared__ __align__(128) unsigned char raw[];
   TrainSmem& sm = *reinterpret_cast<TrainSmem*>(raw);
   const int tid = threadIdx.x, warp = tid >> 5;
-  {
-    const uint4* s1 = reinterpret_cast<const uint4*>(net.fw);
-    uint4* d1 = reinterpret_cast<uint4*>(sm.fw);
-    for (int k = tid; k < FWBYTES / 16; k += TILE) d1[k] = s1[k];
-    const uint4* s2 = reinterpret_cast<const uint4*>(net.bw);
-    uint4* d2 = reinterpret_cast<uint4*>(sm.bw);
-    for (int k = tid; k < BWBYTES / 16; k += TILE) d2[k] = s2[k];
-    for (int k = tid; k < NBIAS; k += TILE) sm.bias[k] = net.bias[k];
-    for (int k = tid; k < NPARAM; k += TILE) sm.acc[k] = 0.0f;
-    if (tid == 0) sm.err = 0;
+  const int row = tid & (TILE - 1), c0 = (tid / TILE) * (HID / 2);  // row of the tile, first of its 32 columns
+  if (tid == 0) {
+    sm.err = 0;
+    tc::mbar_init(&sm.wbar, 1);
   }
   block_setup(&sm.bar, &sm.tmem, TRAIN_TMEM_COLS);
-  const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-  const uint32_t tl = sm.tmem + lane_off;
+  if (tid == 0) {
+    tc::mbar_expect(&sm.wbar, FWBYTES + BWBYTES + NBIAS * sizeof(float));
+    tc::bulk_load(sm.fw, net.fw, FWBYTES, &sm.wbar);
+    tc::bulk_load(sm.bw, net.bw, BWBYTES, &sm.wbar);
+    tc::bulk_load(sm.bias, net.bias, NBIAS * sizeof(float), &sm.wbar);
+  }
+  for (int k = tid; k < NPARAM; k += TRAIN_THREADS) sm.acc[k] = 0.0f;
+  for (int k = tid; k < BPARTS * NBIAS; k += TRAIN_THREADS) (&sm.bacc[0][0])[k] = 0.0f;
+  const uint32_t tl = sm.tmem + ((uint32_t)((warp & 3) * 32) << 16);
   uint32_t phase = 0;
   float lsum = 0.0f;
   // After a timed-out wait (sm.err, seen by every thread after the next barrier) no
@@ -234,20 +249,27 @@ __global__ void __launch_bounds__(TILE, 1) k_train(Net net, const float* __restr
     ++phase;
     tc::fence_after_sync();
   };
+  bool weights = false;
   for (int tile = blockIdx.x; tile * TILE < n; tile += gridDim.x) {
     __syncthreads();  // the previous tile's first-layer weight gradient has read sm.x
     if (sm.err) break;
-    const int r = tile * TILE + tid;
+    const int r = tile * TILE + row;
     const bool valid = r < n;
-    const long long s = valid ? shuffled(first + r, n_all, sa, sc) : 0;
-    float f[IN], t[OUT];
+    float t[OUT];
+    if (c0 == 0) {
+      const long long s = valid ? shuffled(first + r, n_all, sa, sc) : 0;
+      float f[IN];
 #pragma unroll
-    for (int k = 0; k < IN; ++k) f[k] = valid ? X[s * IN + k] : 0.0f;
+      for (int k = 0; k < IN; ++k) f[k] = valid ? X[s * IN + k] : 0.0f;
 #pragma unroll
-    for (int o = 0; o < OUT; ++o) t[o] = valid ? Tg[s * OUT + o] : 0.0f;
-    store_row<IN>(sm.x, tid, f);
+      for (int o = 0; o < OUT; ++o) t[o] = valid ? Tg[s * OUT + o] : 0.0f;
+      store_row<IN>(sm.x, row, f);
+    }
+    if (!weights) {
+      if (!tc::mbar_wait(&sm.wbar, 0)) sm.err = 1;
+      weights = true;
+    }
     // ---- forward: Z(l) kept in TMEM columns 64 (l - 1) -------------------------
-    float y[OUT];
     for (int l = 0; l <= NHID; ++l) {
       tc::fence_smem_to_async();
       __syncthreads();
@@ -261,35 +283,32 @@ __global__ void __launch_bounds__(TILE, 1) k_train(Net net, const float* __restr
       }
       wait_mma();
       if (l < NHID) {
-        const float* b = sm.bias + l * HID;
-#pragma unroll 1
-        for (int c = 0; c < HID; c += 16) {
-          float v[16];
-          tc::tmem_ld16(tl + 64u * l + c, v);
+        const float* b = sm.bias + l * HID + c0;
+        float v[32];
+        tc::tmem_ld32(tl + 64u * l + c0, v);
 #pragma unroll
-          for (int k = 0; k < 16; ++k) v[k] = silu(v[k] + b[c + k]);
-          store_chunk16<HID>(sm.h[l], tid, c, v);
-        }
+        for (int k = 0; k < 32; ++k) v[k] = silu(v[k] + b[k]);
+        store_chunk16<HID>(sm.h[l], row, c0, v);
+        store_chunk16<HID>(sm.h[l], row, c0 + 16, v + 16);
       } else {
+        // ---- loss (mean over samples and outputs) and its gradient -----------------
         float v[16];
-        tc::tmem_ld16(tl + TCOL_Y, v);
+        tc::tmem_ld16(tl + TCOL_Y, v);  // warp-wide loads: unconditional
+        if (c0 == 0) {
+          float g5[16];
 #pragma unroll
-        for (int o = 0; o < OUT; ++o) y[o] = v[o] + sm.bias[NHID * HID + o];
+          for (int o = 0; o < 16; ++o) g5[o] = 0.0f;
+#pragma unroll
+          for (int o = 0; o < OUT; ++o) {
+            const float y = v[o] + sm.bias[NHID * HID + o];
+            const float d = valid ? y - t[o] : 0.0f;
+            lsum += d * d;
+            g5[o] = 2.0f * d * inv_count;
+          }
+          store_chunk16<OUTP>(sm.g5, row, 0, g5);
+        }
       }
       tc::fence_before_sync();
-    }
-    // ---- loss (mean over samples and outputs) and its gradient -------------------
-    {
-      float g5[16];
-#pragma unroll
-      for (int o = 0; o < 16; ++o) g5[o] = 0.0f;
-#pragma unroll
-      for (int o = 0; o < OUT; ++o) {
-        const float d = valid ? y[o] - t[o] : 0.0f;
-        lsum += d * d;
-        g5[o] = 2.0f * d * inv_count;
-      }
-      store_chunk16<OUTP>(sm.g5, tid, 0, g5);
     }
     tc::fence_smem_to_async();
     __syncthreads();
@@ -299,23 +318,21 @@ __global__ void __launch_bounds__(TILE, 1) k_train(Net net, const float* __restr
       issue_wgrad(sm.h[NHID - 1], HID, sm.g5, OUTP, OUTP, sm.tmem + TCOL_Y);
       tc::mma_commit(&sm.bar);
     }
-    add_bias_grad<OUTP, OUT>(sm.acc, P_B5, sm.g5);
+    add_bias_grad<OUTP, OUT>(sm.bacc, NHID * HID, sm.g5);
     wait_mma();
-    add_wgrad<OUTP>(sm.acc, sm.tmem, TCOL_Y, P_W5, OUT);  // warp-wide loads: unconditional
+    if (c0 == 0) add_wgrad<16>(sm.acc, sm.tmem, TCOL_Y, 0, P_W5, OUT);  // whole warps
     tc::fence_before_sync();
     // ---- hidden layers, last to first -------------------------------------------
     for (int l = NHID; l >= 1; --l) {
       __syncthreads();  // the previous bias gradient has finished reading sm.g
-      const float* b = sm.bias + (l - 1) * HID;
-#pragma unroll 1
-      for (int c = 0; c < HID; c += 16) {
-        float dh[16], z[16];
-        tc::tmem_ld16(tl + TCOL_DH + c, dh);
-        tc::tmem_ld16(tl + 64u * (l - 1) + c, z);
+      const float* b = sm.bias + (l - 1) * HID + c0;
+      float dh[32], z[32];
+      tc::tmem_ld32(tl + TCOL_DH + c0, dh);
+      tc::tmem_ld32(tl + 64u * (l - 1) + c0, z);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) dh[k] *= silu_grad(z[k] + b[c + k]);
-        store_chunk16<HID>(sm.g, tid, c, dh);
-      }
+      for (int k = 0; k < 32; ++k) dh[k] *= silu_grad(z[k] + b[k]);
+      store_chunk16<HID>(sm.g, row, c0, dh);
+      store_chunk16<HID>(sm.g, row, c0 + 16, dh + 16);
       tc::fence_before_sync();
       tc::fence_smem_to_async();
       __syncthreads();
@@ -332,18 +349,29 @@ __global__ void __launch_bounds__(TILE, 1) k_train(Net net, const float* __restr
         }
         tc::mma_commit(&sm.bar);
       }
-      add_bias_grad<HID, HID>(sm.acc, l == 1 ? P_B1 : l == 2 ? P_B2 : l == 3 ? P_B3 : P_B4, sm.g);
+      add_bias_grad<HID, HID>(sm.bacc, (l - 1) * HID, sm.g);
       wait_mma();
-      if (l > 1) add_wgrad<HID>(sm.acc, sm.tmem, zcol, l == 2 ? P_W2 : l == 3 ? P_W3 : P_W4, HID);
-      else add_wgrad<IN>(sm.acc, sm.tmem, zcol, P_W1, IN);
+      if (l > 1) add_wgrad<32>(sm.acc, sm.tmem, zcol, c0, l == 2 ? P_W2 : l == 3 ? P_W3 : P_W4, HID);
+      else if (c0 == 0) add_wgrad<16>(sm.acc, sm.tmem, zcol, 0, P_W1, IN);  // whole warps
       tc::fence_before_sync();
     }
   }
   __syncthreads();
-  for (int k = tid; k < NPARAM; k += TILE) atomicAdd(&grad[k], sm.acc[acc_index(k)]);
+  for (int k = tid; k < NPARAM; k += TRAIN_THREADS) {  // biases below: nothing accumulated here
+    const float v = sm.acc[k];
+    if (v != 0.0f) atomicAdd(&grad[k], v);
+  }
+  for (int k = tid; k < NHID * HID + OUT; k += TRAIN_THREADS) {
+    float v = sm.bacc[0][k];
+#pragma unroll
+    for (int q = 1; q < BPARTS; ++q) v += sm.bacc[q][k];
+    const int l = k / HID;  // layer l's biases follow its weights
+    atomicAdd(&grad[(l == 0 ? P_B1 : l == 1 ? P_B2 : l == 2 ? P_B3 : l == 3 ? P_B4 : P_B5) + k - l * HID], v);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((tid & 31) == 0) atomicAdd(loss, (double)lsum);
+  if ((tid & 31) == 0 && c0 == 0) atomicAdd(loss, (double)lsum);
+  if (!weights || sm.err) tc::mbar_wait(&sm.wbar, 0);  // no copy is left in flight
   drain_after_timeout(&sm.bar, sm.err, phase);
   block_teardown(sm.tmem, TRAIN_TMEM_COLS);
   if (tid == 0 && sm.err) atomicExch(err, 1);
@@ -397,7 +425,8 @@ struct rw_mlp {
   int device = 0;
   cudaStream_t st = nullptr;
   float* params = nullptr;  // FP32 master
-  float* grad = nullptr;
+  float* grad = nullptr;  // as the training kernel accumulates it (acc_index)
+  float* gord = nullptr;  // in parameter order
   float* m = nullptr;
   float* v = nullptr;
   unsigned char* fw = nullptr;
@@ -483,7 +512,7 @@ rw_status grad_dev(rw_mlp* m, const float* dx, const float* dt, long long n_all,
   MLP_CU(m, cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int tiles = (n + TILE - 1) / TILE;
   const int grid = std::min(tiles, num_sms(m->device));
-  k_train<<<grid, TILE, smem, m->st>>>(net_of(m), dx, dt, n_all, first, n, sa, sc, inv_count, m->grad, m->loss,
+  k_train<<<grid, TRAIN_THREADS, smem, m->st>>>(net_of(m), dx, dt, n_all, first, n, sa, sc, inv_count, m->grad, m->loss,
                                        m->err);
   MLP_CU(m, cudaGetLastError());
   return RW_OK;
@@ -558,6 +587,7 @@ rw_status rw_mlp_create(int device, uint64_t seed, int64_t sample_capacity, rw_m
     return bad(fail(nullptr, RW_ECUDA, "rw_mlp_create: stream"));
   bool ok = cudaMalloc(&m->params, NPARAM * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&m->grad, NPARAM * sizeof(float)) == cudaSuccess &&
+            cudaMalloc(&m->gord, NPARAM * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&m->m, NPARAM * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&m->v, NPARAM * sizeof(float)) == cudaSuccess && cudaMalloc(&m->fw, FWBYTES) == cudaSuccess &&
             cudaMalloc(&m->bw, BWBYTES) == cudaSuccess &&
@@ -601,7 +631,7 @@ rw_status rw_mlp_destroy(rw_mlp* m) {
   if (!m) return RW_OK;
   cudaSetDevice(m->device);
   if (m->st) cudaStreamSynchronize(m->st);
-  for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->m, (void*)m->v, (void*)m->fw, (void*)m->bw,
+  for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->gord, (void*)m->m, (void*)m->v, (void*)m->fw, (void*)m->bw,
                   (void*)m->bias, (void*)m->err, (void*)m->loss, (void*)m->ranges, (void*)m->sx, (void*)m->stg, (void*)m->ws})
     if (p) cudaFree(p);
   if (m->st) cudaStreamDestroy(m->st);
@@ -666,7 +696,9 @@ rw_status rw_mlp_grad(rw_mlp* m, const float* x, const float* t, int64_t n, doub
     if (s == RW_OK) s = check_err(m);
     if (s == RW_OK) {
       double l = 0.0;
-      MLP_CU(m, cudaMemcpyAsync(grad, m->grad, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+      k_grad_order<<<(NPARAM + 255) / 256, 256, 0, m->st>>>(m->grad, m->gord);
+      MLP_CU(m, cudaGetLastError());
+      MLP_CU(m, cudaMemcpyAsync(grad, m->gord, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->st));
       MLP_CU(m, cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
       MLP_CU(m, cudaMemsetAsync(m->grad, 0, NPARAM * sizeof(float), m->st));
       MLP_CU(m, cudaStreamSynchronize(m->st));
