@@ -501,6 +501,12 @@ template <class T> struct Engine final : EngineBase {
                                (int)sizeof(Ix2Smem<T>)));
     RW_CU(cudaFuncSetAttribute(k_interaction2<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(Ix2Smem<T>)));
+    if constexpr (kStages) {
+      RW_CU(cudaFuncSetAttribute(k_predictor<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 256 * staged_row_bytes<T>(0, true)));
+      RW_CU(cudaFuncSetAttribute(k_corrector<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 256 * staged_row_bytes<T>(1, true)));
+    }
     for (auto* f : {k_rs_downsweep<4>, k_rs_downsweep<8>, k_rs_downsweep<16>})
       RW_CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)rs_down_smem(1 << RS_MAX_BITS, 16 * RS_THREADS)));
@@ -692,14 +698,27 @@ template <class T> struct Engine final : EngineBase {
     }
     cpar ^= 1;
   }
+  // The FP32 predictor reads staged rows at every size (never slower from 700 to 1.9M particles:
+  // 13.7 -> 12.7 us at 56k, 55 -> 51 at 557k, 172 -> 140 at 1.9M); the corrector, whose loads
+  // are all issued early anyway, where the rows no longer fit in L2 (56k: 14.3 direct, 15.3
+  // staged; 335k: 38 and 42; 0.8M: 72.8 and 71.9; 1.1M: 92.5 and 86.2; 1.9M: 175 and 150).
+  // FP64 rows are read directly (60k: 18.9 and 17.5 us, staged 21.8 and 24.9).
+  static constexpr bool kStages = sizeof(T) == 4;
+  static constexpr int kStagedCorrector = 800000;
   void predictor() override {
     if (P.closure) return integrate_closure(0);
-    k_predictor<T><<<nblk(P.np, integ_threads), integ_threads, 0, st>>>(P, S, d_dyn);
+    const int smem = kStages ? integ_threads * staged_row_bytes<T>(0, P.mixed != 0) : 0;
+    k_predictor<T, kStages><<<nblk(P.np, integ_threads), integ_threads, smem, st>>>(P, S, d_dyn);
     check_launch();
   }
   void corrector() override {
     if (P.closure) return integrate_closure(1);
-    k_corrector<T><<<nblk(P.npb + P.npm0, integ_threads), integ_threads, 0, st>>>(P, S, d_dyn);
+    const unsigned grid = nblk(P.npb + P.npm0, integ_threads);
+    if (kStages && P.np >= kStagedCorrector)
+      k_corrector<T, kStages>
+          <<<grid, integ_threads, integ_threads * staged_row_bytes<T>(1, P.mixed != 0), st>>>(P, S, d_dyn);
+    else
+      k_corrector<T, false><<<grid, integ_threads, 0, st>>>(P, S, d_dyn);
     check_launch();
   }
   // An integrator stage with the learned closure: one persistent launch, four 128-thread

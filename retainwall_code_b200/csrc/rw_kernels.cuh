@@ -2618,43 +2618,135 @@ template <class T, bool Strict> __global__ void __launch_bounds__(IX2_TB) k_inte
 }
 
 // ---------------------------------------------------------------------------------
+// What an integrator reads of its rows: the state's own arrays (row i at [i]) or a block's
+// rows staged in shared memory (row of thread t at [t]).
+// ---------------------------------------------------------------------------------
+template <class T> struct RowIn {
+  const V4<T>*pos, *vel, *sa, *na;  // predictor: the state; corrector: the step-start state
+  const V4<T>*idm, *acc, *da, *spin, *po, *kp, *kv;
+  const V2<T>*sb, *nb, *db;
+  const int4 *codes, *cell;
+  const float* dacc;
+};
+template <class T, int Stage> RWD RowIn<T> row_in(const DevState<T>& S, const Dyn<T>* dyn) {
+  const int c = dyn->cur_main, ci = dyn->cur_ini;
+  RowIn<T> r;
+  r.pos = Stage == 0 ? S.pos[c] : S.pos_ini[ci];
+  r.vel = Stage == 0 ? S.vel[c] : S.vel_ini[ci];
+  r.sa = Stage == 0 ? S.str_a[c] : S.stri_a[ci];
+  r.sb = Stage == 0 ? S.str_b[c] : S.stri_b[ci];
+  r.na = Stage == 0 ? S.stn_a[c] : S.stni_a[ci];
+  r.nb = Stage == 0 ? S.stn_b[c] : S.stni_b[ci];
+  r.kp = Stage == 0 ? S.cmp_p[c] : S.cmp_pi[ci];
+  r.kv = Stage == 0 ? S.cmp_v[c] : S.cmp_vi[ci];
+  r.idm = S.idm[c];
+  r.acc = S.accad;
+  r.da = S.ace_a;
+  r.db = S.ace_b;
+  r.spin = S.spin;
+  r.codes = S.codes[c];
+  r.cell = S.cellpos[c];
+  r.po = S.pos_ori[c];
+  r.dacc = S.dacc[dyn->lbuf];
+  return r;
+}
+// Bytes a staged row takes.
+template <class T> constexpr int staged_row_bytes(int stage, bool mixed) {
+  const int v4 = 8 + (stage == 1) + (mixed ? 2 : 0);
+  return v4 * (int)sizeof(V4<T>) + 3 * (int)sizeof(V2<T>) + (1 + (stage == 1)) * (int)sizeof(int4) + (int)sizeof(float);
+}
+// Fetches the block's rows [i0, i0 + blockDim.x) into shared memory with one bulk copy per
+// array and points `in` at them; false if they did not arrive (the caller then reads the
+// state's arrays, and waits once more before it ends).  Every array starts on a 256-byte
+// boundary and i0 is a multiple of the block, so a copy starts and ends on 16 bytes.
+template <class T, int Stage>
+RWD bool stage_rows(const Params<T>& P, int i0, unsigned char* raw, uint64_t* bar, RowIn<T>& in) {
+  const int nt = blockDim.x;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_expect(bar, (uint32_t)(nt * staged_row_bytes<T>(Stage, P.mixed != 0)));
+  }
+  int off = 0;
+  auto put = [&](auto*& p) {
+    const int bytes = nt * (int)sizeof(*p);
+    if (threadIdx.x == 0) tc::bulk_load(raw + off, p + i0, (uint32_t)bytes, bar);
+    p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(raw + off);
+    off += bytes;
+  };
+  put(in.pos);
+  put(in.vel);
+  put(in.codes);
+  put(in.sa);
+  put(in.na);
+  put(in.acc);
+  put(in.da);
+  put(in.spin);
+  put(in.idm);
+  if (Stage == 1) {
+    put(in.cell);
+    put(in.po);
+  }
+  if (P.mixed) {
+    put(in.kp);
+    put(in.kv);
+  }
+  put(in.sb);
+  put(in.nb);
+  put(in.db);
+  put(in.dacc);
+  __syncthreads();
+  return __syncthreads_and(tc::mbar_wait(bar, 0));
+}
+
+// ---------------------------------------------------------------------------------
 // Predictor (src/predictor_corrector.cu:52-103): saves the step-start state into the
 // *_ini buffers (the reference's four D2D copies) and advances material half a step.
 // ---------------------------------------------------------------------------------
-// Both integrators are held to four 256-thread blocks per SM (64 registers, about
-// 100 spilled bytes): they stream about 300 B per particle, and at the two blocks
-// their natural 94 registers allow they wait on memory (measured 19% faster at
-// three blocks, another 5% at four).
+// Both integrators stream about 400 B per particle.  Read directly, the predictor waits on
+// memory in four dependent turns (its step-start stores hold the later loads back): four
+// 256-thread blocks per SM, 64 registers, 172 us at 1.9M particles, 4.6 TB/s.  With its rows
+// staged by bulk copies it waits once, the step-start copies leave from shared memory, and
+// three blocks (80 registers, 32 spilled bytes) take 140 us, 5.7 TB/s (four blocks: 149, two
+// without spills: 170); fetching the next blocks' rows into L2 ahead only adds (152).
 // In FP64 four blocks spill 500 to 800 bytes; two (128 registers) take 18 us instead of 26 at
 // 60k particles and 28 instead of 31 to 33 at 112k (three: 23 and 28, one: 23 and 34).
-// One row of the predictor.  With the learned closure on, HypoCS rows keep their stress
-// here and the closure's pass updates it (and writes their record).
-template <class T> RWD void predictor_row(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i) {
+// One row of the predictor, read at in[k]; Saved: the step-start copies are made elsewhere.
+// With the learned closure on, HypoCS rows keep their stress here and the closure's pass
+// updates it (and writes their record).
+template <bool Saved, class T>
+RWD void predictor_row(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i, const RowIn<T>& in, int k) {
   if (i >= P.np) return;
   const int c = dyn->cur_main, ci = dyn->cur_ini;
   const int npm = dyn->npm;
-  V4<T> ps = S.pos[c][i];
-  V4<T> vr = S.vel[c][i];
-  S.pos_ini[ci][i] = ps;
-  S.vel_ini[ci][i] = vr;
+  V4<T> ps = in.pos[k];
+  V4<T> vr = in.vel[k];
+  if (!Saved) {
+    S.pos_ini[ci][i] = ps;
+    S.vel_ini[ci][i] = vr;
+  }
   V4<T> kp{T(0), T(0), T(0), T(0)}, kv{T(0), T(0), T(0), T(0)};
   if (P.mixed) {
-    kp = S.cmp_p[c][i];
-    kv = S.cmp_v[c][i];
-    S.cmp_pi[ci][i] = kp;
-    S.cmp_vi[ci][i] = kv;
+    kp = in.kp[k];
+    kv = in.kv[k];
+    if (!Saved) {
+      S.cmp_pi[ci][i] = kp;
+      S.cmp_vi[ci][i] = kv;
+    }
   }
   if (npm == 0 || i >= P.npb + npm) return;
-  S6<T> sg = ld6(S.str_a[c], S.str_b[c], i);
-  S6<T> sn = ld6(S.stn_a[c], S.stn_b[c], i);
-  st6(S.stri_a[ci], S.stri_b[ci], i, sg);
-  st6(S.stni_a[ci], S.stni_b[ci], i, sn);
+  S6<T> sg = ld6(in.sa, in.sb, k);
+  S6<T> sn = ld6(in.na, in.nb, k);
+  if (!Saved) {
+    st6(S.stri_a[ci], S.stri_b[ci], i, sg);
+    st6(S.stni_a[ci], S.stni_b[ci], i, sn);
+  }
   if (i < P.npb) return;
-  const int4 code = S.codes[c][i];
+  const int4 code = in.codes[k];
   if (code.y != 1) return;
-  const T mass = S.idm[c][i].y;  // for the neighbour record (read early: the stores below may alias)
+  const T mass = in.idm[k].y;  // for the neighbour record (read early: the stores below may alias)
   const T hdt = T(0.5f) * P.dt;
-  const V4<T> acc = S.accad[i];
+  const V4<T> acc = in.acc[k];
   if (P.mixed) {  // compensated half step; the compensation itself is not kept
     kahan_add(vr.x, kv.x, acc.x * hdt);
     kahan_add(vr.y, kv.y, acc.y * hdt);
@@ -2669,18 +2761,18 @@ template <class T> RWD void predictor_row(const Params<T>& P, const DevState<T>&
   }
   {  // distance since the lists were built, after this half step
     const float a = (float)(f_sqrt(vr.x * vr.x + vr.y * vr.y + vr.z * vr.z) * hdt);
-    if (S.dacc[dyn->lbuf][i] + a + P.disp_eps > P.disp_lim) const_cast<Dyn<T>*>(dyn)->list_kill = 1;
+    if (in.dacc[k] + a + P.disp_eps > P.disp_lim) const_cast<Dyn<T>*>(dyn)->list_kill = 1;
   }
   const T* mp = P.model_par[code.w];
   vr.w = f_max(vr.w, mp[kMatSize - 2]);
   vr.w = f_min(vr.w, mp[kMatSize - 1]);
-  const S6<T> D = ld6(S.ace_a, S.ace_b, i);
+  const S6<T> D = ld6(in.da, in.db, k);
   sn = sn + D * hdt;
   bool yld = false;
   T mcrt = T(0);
   const bool by_closure = P.closure && code.z == RW_MODEL_HYPO_CS;  // the closure pass updates the stress
   const HypoC<T> hc = P.hypo[code.w];
-  if (!by_closure) constitutive(code.z, mp, hdt, vr.w, xyz(S.spin[i]), D, sg, yld, mcrt, P.mixed != 0, &hc);
+  if (!by_closure) constitutive(code.z, mp, hdt, vr.w, xyz(in.spin[k]), D, sg, yld, mcrt, P.mixed != 0, &hc);
   S.pos[c][i] = ps;
   S.vel[c][i] = vr;
   st6(S.stn_a[c], S.stn_b[c], i, sn);
@@ -2689,9 +2781,39 @@ template <class T> RWD void predictor_row(const Params<T>& P, const DevState<T>&
   if (!by_closure) write_rec(P, S.rec, i, ps, vr, sg, mass, code.x >= 10);
 }
 
-template <class T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_predictor(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
-  predictor_row(P, S, dyn, blockIdx.x * blockDim.x + threadIdx.x);
+template <class T, bool Staged>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? (Staged ? 3 : 4) : 2)
+    k_predictor(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
+  const int i0 = blockIdx.x * blockDim.x, tid = threadIdx.x;
+  const RowIn<T> in = row_in<T, 0>(S, dyn);
+  if constexpr (Staged) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    __shared__ uint64_t bar;
+    if (i0 >= P.npb && i0 + (int)blockDim.x <= P.npb + dyn->npm) {  // block-uniform
+      RowIn<T> st = in;
+      if (stage_rows<T, 0>(P, i0, raw, &bar, st)) {
+        if (tid == 0) {  // the step-start copies leave from the staged rows
+          const int ci = dyn->cur_ini, n4 = blockDim.x * (int)sizeof(V4<T>), n2 = blockDim.x * (int)sizeof(V2<T>);
+          tc::bulk_store(S.pos_ini[ci] + i0, st.pos, n4);
+          tc::bulk_store(S.vel_ini[ci] + i0, st.vel, n4);
+          tc::bulk_store(S.stri_a[ci] + i0, st.sa, n4);
+          tc::bulk_store(S.stri_b[ci] + i0, st.sb, n2);
+          tc::bulk_store(S.stni_a[ci] + i0, st.na, n4);
+          tc::bulk_store(S.stni_b[ci] + i0, st.nb, n2);
+          if (P.mixed) {
+            tc::bulk_store(S.cmp_pi[ci] + i0, st.kp, n4);
+            tc::bulk_store(S.cmp_vi[ci] + i0, st.kv, n4);
+          }
+          tc::bulk_store_commit();
+        }
+        predictor_row<true>(P, S, dyn, i0 + tid, st, tid);
+        if (tid == 0) tc::bulk_store_wait();
+        return;
+      }
+      tc::mbar_wait(&bar, 0);  // late: read the arrays instead, with no copy left in flight
+    }
+  }
+  predictor_row<false>(P, S, dyn, i0 + tid, in, i0 + tid);
 }
 
 // ---------------------------------------------------------------------------------
@@ -2724,11 +2846,10 @@ template <class T> RWD void mark_cell(const Params<T>& P, const DevState<T>& S, 
 // must stay within the skin's share, else every list is rebuilt.  A cell change marks
 // both cells (the next list update rebuilds the lists around them); leaving the grid
 // (deletion) makes it a full build.
-template <class T> RWD void list_account(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i, float step,
-                                         I3 from, I3 to) {
-  float* dacc = S.dacc[dyn->lbuf];
-  const float d = dacc[i] + step + P.disp_eps;
-  dacc[i] = d;
+template <class T> RWD void list_account(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i, float dacc,
+                                         float step, I3 from, I3 to) {
+  const float d = dacc + step + P.disp_eps;
+  S.dacc[dyn->lbuf][i] = d;
   Dyn<T>* w = const_cast<Dyn<T>*>(dyn);
   if (from.x != to.x || from.y != to.y || from.z != to.z) {
     w->cells_dirty = 1;
@@ -2744,18 +2865,19 @@ template <class T> RWD void list_account(const Params<T>& P, const DevState<T>& 
 
 // One row of the corrector (moving boundary rows and soil rows); with the learned
 // closure on, HypoCS rows keep their stress here, as in predictor_row.
-template <class T> RWD void corrector_row(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i) {
+template <class T>
+RWD void corrector_row(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int i, const RowIn<T>& in, int k) {
   const int npm = dyn->npm;
   if (i >= P.npb + npm) return;
-  const int c = dyn->cur_main, ci = dyn->cur_ini;
-  const int4 code = S.codes[c][i];
+  const int c = dyn->cur_main;
+  const int4 code = in.codes[k];
   if (code.y != 1) return;
   const T th = P.two_h;
   if (i < P.npb) {
     if (P.n_motion <= 0) return;
     const Motion<T>& mv = dyn->mv[code.w];
     V3<T> vel{mv.trans_vel.x, mv.trans_vel.y, mv.trans_vel.z};
-    int4 cp = S.cellpos[c][i];
+    int4 cp = in.cell[k];
     if (mv.is_rotat && mv.pattern != RW_PATTERN_CIRCLE) {
       const V3<T> pabs = ld3(S.pos[c], i) + mulI(I3{cp.x, cp.y, cp.z}, th);
       const V3<T> rp{mv.pos_rp.x, mv.pos_rp.y, mv.pos_rp.z};
@@ -2767,35 +2889,35 @@ template <class T> RWD void corrector_row(const Params<T>& P, const DevState<T>&
       const V3<T> n = dotFV(R, xyz(n4));
       S.normal[cn][i] = v4(n, n4.w);
     }
-    V4<T> ps = add3(S.pos_ini[ci][i], vel * P.dt);
+    V4<T> ps = add3(in.pos[k], vel * P.dt);
     const I3 dc = rebin(ps, th);
     S.pos[c][i] = ps;
     S.cellpos[c][i] = int4{cp.x + dc.x, cp.y + dc.y, cp.z + dc.z, cp.w};
-    list_account(P, S, dyn, i, (float)(f_sqrt(dot(vel, vel)) * P.dt), I3{cp.x, cp.y, cp.z},
+    list_account(P, S, dyn, i, in.dacc[k], (float)(f_sqrt(dot(vel, vel)) * P.dt), I3{cp.x, cp.y, cp.z},
                  I3{cp.x + dc.x, cp.y + dc.y, cp.z + dc.z});
     return;
   }
-  const V4<T> vri = S.vel_ini[ci][i];
-  V4<T> id = S.idm[c][i];  // read early: the stores below may alias
+  const V4<T> vri = in.vel[k];
+  V4<T> id = in.idm[k];  // read early: the stores below may alias
   V4<T> vr, ps;
   V4<T> kp{T(0), T(0), T(0), T(0)}, kv{T(0), T(0), T(0), T(0)};
   if (P.mixed) {  // compensated full step (position and velocity keep their lost low bits)
-    kp = S.cmp_pi[ci][i];
-    kv = S.cmp_vi[ci][i];
-    const V4<T> acc = S.accad[i];
+    kp = in.kp[k];
+    kv = in.kv[k];
+    const V4<T> acc = in.acc[k];
     vr = vri;
     kahan_add(vr.x, kv.x, acc.x * P.dt);
     kahan_add(vr.y, kv.y, acc.y * P.dt);
     kahan_add(vr.z, kv.z, acc.z * P.dt);
     kahan_add(vr.w, kv.w, acc.w * P.dt);
-    ps = S.pos_ini[ci][i];
+    ps = in.pos[k];
     const T hdt = T(0.5f) * P.dt;
     kahan_add(ps.x, kp.x, (vr.x + vri.x) * hdt);
     kahan_add(ps.y, kp.y, (vr.y + vri.y) * hdt);
     kahan_add(ps.z, kp.z, (vr.z + vri.z) * hdt);
   } else {
-    vr = vri + S.accad[i] * P.dt;
-    ps = add3(S.pos_ini[ci][i], xyz(vr + vri) * (T(0.5f) * P.dt));
+    vr = vri + in.acc[k] * P.dt;
+    ps = add3(in.pos[k], xyz(vr + vri) * (T(0.5f) * P.dt));
   }
   const T* mp = P.model_par[code.w];
   vr.w = f_max(vr.w, mp[kMatSize - 2]);
@@ -2810,28 +2932,28 @@ template <class T> RWD void corrector_row(const Params<T>& P, const DevState<T>&
     S.cmp_p[c][i] = kp;
     S.cmp_v[c][i] = kv;
   }
-  const int4 cp0 = S.cellpos[c][i];
+  const int4 cp0 = in.cell[k];
   int4 cp = int4{cp0.x + dc.x, cp0.y + dc.y, cp0.z + dc.z, cp0.w};
   if (P.periodbound) period_wrap(P, cp, ps);
   {
     const V3<T> inc = xyz(vr + vri) * (T(0.5f) * P.dt);
-    list_account(P, S, dyn, i, (float)f_sqrt(dot(inc, inc)), I3{cp0.x, cp0.y, cp0.z}, I3{cp.x, cp.y, cp.z});
+    list_account(P, S, dyn, i, in.dacc[k], (float)f_sqrt(dot(inc, inc)), I3{cp0.x, cp0.y, cp0.z}, I3{cp.x, cp.y, cp.z});
   }
-  S6<T> sg = ld6(S.stri_a[ci], S.stri_b[ci], i);
-  const S6<T> D = ld6(S.ace_a, S.ace_b, i);
-  const S6<T> sn = ld6(S.stni_a[ci], S.stni_b[ci], i) + D * P.dt;
+  S6<T> sg = ld6(in.sa, in.sb, k);
+  const S6<T> D = ld6(in.da, in.db, k);
+  const S6<T> sn = ld6(in.na, in.nb, k) + D * P.dt;
   bool yld = false;
   T mcrt = T(0);
   const bool by_closure = P.closure && code.z == RW_MODEL_HYPO_CS;  // the closure pass updates the stress
   const HypoC<T> hc = P.hypo[code.w];
-  if (!by_closure) constitutive(code.z, mp, P.dt, vr.w, xyz(S.spin[i]), D, sg, yld, mcrt, P.mixed != 0, &hc);
+  if (!by_closure) constitutive(code.z, mp, P.dt, vr.w, xyz(in.spin[k]), D, sg, yld, mcrt, P.mixed != 0, &hc);
   if (!yld) id.x = T(100);
   id.w = mcrt;
   if (!in_grid(P, I3{cp.x, cp.y, cp.z})) {
     cp.w = P.ncell_delete_m;
     id.x = T(999.0);
   }
-  V4<T> po = S.pos_ori[c][i];
+  V4<T> po = in.po[k];
   if (dyn->time_f <= P.dt) po = V4<T>{T(0), T(0), T(0), T(0)};
   po = add3(po, xyz(vr) * P.dt);
   S.vel[c][i] = vr;
@@ -2845,9 +2967,24 @@ template <class T> RWD void corrector_row(const Params<T>& P, const DevState<T>&
   if (!by_closure) write_rec(P, S.rec, i, ps, vr, sg, id.y, code.x >= 10);
 }
 
-template <class T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_corrector(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
-  corrector_row(P, S, dyn, blockIdx.x * blockDim.x + threadIdx.x);
+template <class T, bool Staged>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? (Staged ? 3 : 4) : 2)
+    k_corrector(const Params<T> P, DevState<T> S, const Dyn<T>* dyn) {
+  const int i0 = blockIdx.x * blockDim.x, tid = threadIdx.x;
+  const RowIn<T> in = row_in<T, 1>(S, dyn);
+  if constexpr (Staged) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    __shared__ uint64_t bar;
+    if (i0 >= P.npb && i0 + (int)blockDim.x <= P.npb + dyn->npm) {  // block-uniform
+      RowIn<T> st = in;
+      if (stage_rows<T, 1>(P, i0, raw, &bar, st)) {
+        corrector_row(P, S, dyn, i0 + tid, st, tid);
+        return;
+      }
+      tc::mbar_wait(&bar, 0);
+    }
+  }
+  corrector_row(P, S, dyn, i0 + tid, in, i0 + tid);
 }
 
 // ---------------------------------------------------------------------------------
@@ -3364,19 +3501,20 @@ __global__ void __launch_bounds__(mlp::TILE) k_integrate_cl(const Params<T> P, D
   const int soil_rows = Stage == 0 ? P.np - P.npb : dyn->npm;
   const int n_tiles = nb_tiles + (soil_rows + mlp::TILE - 1) / mlp::TILE;
   uint32_t phase = 0;
+  const RowIn<T> in = row_in<T, Stage>(S, dyn);
   for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {  // block-uniform
     if (tile < nb_tiles) {
       const int i = tile * mlp::TILE + threadIdx.x;
       if (i < P.npb) {
-        if (Stage == 0) predictor_row(P, S, dyn, i);
-        else corrector_row(P, S, dyn, i);
+        if (Stage == 0) predictor_row<false>(P, S, dyn, i, in, i);
+        else corrector_row(P, S, dyn, i, in, i);
       }
       continue;
     }
     const int st = tile - nb_tiles, t = st * mlp::TILE + threadIdx.x;
     if (t < soil_rows) {
-      if (Stage == 0) predictor_row(P, S, dyn, P.npb + t);
-      else corrector_row(P, S, dyn, P.npb + t);
+      if (Stage == 0) predictor_row<false>(P, S, dyn, P.npb + t, in, P.npb + t);
+      else corrector_row(P, S, dyn, P.npb + t, in, P.npb + t);
     }
     closure_tile(P, S, dyn, sm, tr, stats, Stage, st, phase);
   }
