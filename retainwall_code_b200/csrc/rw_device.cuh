@@ -299,9 +299,10 @@ template <class T> struct HypoPre {
   HypoC<T> c;
 };
 
-// false: the zero-stress reset branch (I1 > -4) was taken and sigma is final.
+// false: the zero-stress reset branch (I1 > -4) was taken and sigma is final.  state: e, e_crt
+// and fd where they are known already (density is then not read).
 template <class T> RWD bool hypo_cs_pre(T density, V3<T> om, S6<T> D, S6<T>& sigma, const T* mp, T& M_crt, bool dnorm,
-                                        HypoPre<T>& h, const HypoC<T>* pre = nullptr) {
+                                        HypoPre<T>& h, const HypoC<T>* pre = nullptr, const V3<T>* state = nullptr) {
   T coh = mp[3], p_ref = mp[4], void_co = mp[5], lambda = mp[6];
   T xi = mp[7], alpha = mp[8], void_min = mp[9], void_max = mp[10], void_0 = mp[11], rho0 = mp[12];
   h.c = hypo_coef(mp, pre);
@@ -321,6 +322,13 @@ template <class T> RWD bool hypo_cs_pre(T density, V3<T> om, S6<T> D, S6<T>& sig
   h.tr_sD = trace2(h.str, D);
   h.nD = rate_norm(D, dnorm);
   h.p = (T)(-(double)I1 / 3.0);
+  if (state) {
+    h.e = state->x;
+    h.e_crt = state->y;
+    h.fd = state->z;
+    M_crt = h.e - h.e_crt;
+    return true;
+  }
   T e = (T)((1.0 + (double)void_0) * (double)rho0 / (double)density - 1.0);
   e = f_max(e, void_min);
   h.e = f_min(e, void_max);

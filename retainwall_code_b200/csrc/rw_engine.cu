@@ -721,16 +721,17 @@ template <class T> struct Engine final : EngineBase {
       k_corrector<T, false><<<grid, integ_threads, 0, st>>>(P, S, d_dyn);
     check_launch();
   }
-  // An integrator stage with the learned closure: one persistent launch, four 128-thread
-  // blocks per SM, each looping over tiles of rows (k_integrate_cl).
+  // An integrator stage with the learned closure: one persistent launch whose groups of 128
+  // threads loop over tiles of rows (k_integrate_cl).
   void integrate_closure(int stage) {
     const long tiles = nblk(P.npb, mlp::TILE) + nblk(P.np - P.npb, mlp::TILE);
-    const unsigned grid = (unsigned)std::max(1L, std::min(tiles, 4L * nsm));
+    constexpr int kG = kClGroups<T>, smem = (int)sizeof(mlp::FwdSmem<kG>);
+    const unsigned grid = (unsigned)std::max(1L, std::min((tiles + kG - 1) / kG, (long)kClBlocks<T> * nsm));
     const mlp::Net net = mlp::net_view(cl_net);
     if (stage == 0)
-      k_integrate_cl<T, 0><<<grid, mlp::TILE, sizeof(mlp::FwdSmem), st>>>(P, S, d_dyn, net, cl_trust, d_clstats);
+      k_integrate_cl<T, 0><<<grid, kG * mlp::TILE, smem, st>>>(P, S, d_dyn, net, cl_trust, d_clstats);
     else
-      k_integrate_cl<T, 1><<<grid, mlp::TILE, sizeof(mlp::FwdSmem), st>>>(P, S, d_dyn, net, cl_trust, d_clstats);
+      k_integrate_cl<T, 1><<<grid, kG * mlp::TILE, smem, st>>>(P, S, d_dyn, net, cl_trust, d_clstats);
     check_launch();
   }
 
@@ -764,9 +765,9 @@ template <class T> struct Engine final : EngineBase {
     cl_trust.err_max = (float)cl_err_max;
     RW_CU(cudaSetDevice(device));
     RW_CU(cudaFuncSetAttribute(k_integrate_cl<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(mlp::FwdSmem)));
+                               (int)sizeof(mlp::FwdSmem<kClGroups<T>>)));
     RW_CU(cudaFuncSetAttribute(k_integrate_cl<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(mlp::FwdSmem)));
+                               (int)sizeof(mlp::FwdSmem<kClGroups<T>>)));
     RW_CU(cudaMemsetAsync(d_clstats, 0, 4 * sizeof(double), st));
     RW_CU(cudaStreamSynchronize(st));
     P.closure = 1;

@@ -3386,13 +3386,14 @@ template <class T> __global__ void k_collect(const Params<T> P, DevState<T> S, c
 // the Jaumann term, the cut-offs and every particle outside the trust region (or whose
 // output leaves it) stay exact.  Every closure update is judged against the exact rate:
 // stats = [offered, used, sum of relative errors, largest relative error].
-// One tile of 128 soil slots (t = tile * 128 + thread); every thread of the block calls
-// it for the same tile (the network runs on the whole tile).
+// One tile of 128 soil slots; every thread of the group calls it for the same tile (the
+// network runs on the whole tile).
 template <class T>
-RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, mlp::FwdSmem& sm,
-                      const ClosureTrust& tr, double* stats, int stage, int tile, uint32_t& phase) {
+RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, const mlp::FwdWeights& w,
+                      mlp::FwdTile& ft, int g, const ClosureTrust& tr, double* stats, int stage, int tile,
+                      uint32_t& phase) {
   const int npm = dyn->npm, c = dyn->cur_main;
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x & (mlp::TILE - 1), lane = tid & 31;
   const T dt = stage == 0 ? T(0.5f) * P.dt : P.dt;
   {
     const int t = tile * mlp::TILE + tid, i = P.npb + t;
@@ -3401,6 +3402,7 @@ RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dy
 #pragma unroll
     for (int k = 0; k < mlp::IN; ++k) f[k] = 0.0f;
     int4 code{0, 0, 0, 0};
+    V3<T> vs{T(0), T(0), T(0)};  // e, e_c and the void-ratio factor (two powers), kept for the update
     if (t < npm) {
       code = S.codes[c][i];
       mine = code.y == 1 && code.z == RW_MODEL_HYPO_CS;
@@ -3411,8 +3413,9 @@ RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dy
         HypoPre<T> h;
         T mcrt;
         const HypoC<T> hc = P.hypo[code.w];
-        if (hypo_cs_pre(S.vel[c][i].w, V3<T>{T(0), T(0), T(0)}, D, sg, mp, mcrt, P.mixed != 0, h, &hc) &&
-            h.nD > T(0)) {
+        const bool pre = hypo_cs_pre(S.vel[c][i].w, V3<T>{T(0), T(0), T(0)}, D, sg, mp, mcrt, P.mixed != 0, h, &hc);
+        if (pre) vs = V3<T>{h.e, h.e_crt, h.fd};
+        if (pre && h.nD > T(0)) {
           closure_features(h, D, mp, f);
           act = true;
 #pragma unroll
@@ -3426,9 +3429,13 @@ RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dy
     float y[mlp::OUT];
 #pragma unroll
     for (int o = 0; o < mlp::OUT; ++o) y[o] = 0.0f;
-    if (__syncthreads_or(act)) {  // a tile without a trusted particle skips the network
-      mlp::store_row<mlp::IN>(sm.x, tid, f);
-      mlp::forward_tile(sm, 0, phase, y);
+    ft.any = 0;
+    mlp::group_sync(g);
+    if (act) ft.any = 1;
+    mlp::group_sync(g);
+    if (ft.any) {  // a tile without a trusted particle skips the network
+      mlp::store_row<mlp::IN>(ft.h, tid, f);
+      mlp::forward_tile(w, ft, g, phase, y);
     }
     float used = 0.0f, offered = 0.0f, err = 0.0f;
     if (mine) {
@@ -3439,9 +3446,9 @@ RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dy
       HypoPre<T> h;
       T mcrt = T(0);
       const HypoC<T> hc = P.hypo[code.w];
-      if (hypo_cs_pre(S.vel[c][i].w, V3<T>{om4.x, om4.y, om4.z}, D, sg, mp, mcrt, P.mixed != 0, h, &hc)) {
+      if (hypo_cs_pre(T(0), V3<T>{om4.x, om4.y, om4.z}, D, sg, mp, mcrt, P.mixed != 0, h, &hc, &vs)) {
         S6<T> rate;
-        bool use = act && !sm.err;
+        bool use = act && !ft.err;
 #pragma unroll
         for (int o = 0; o < mlp::OUT; ++o) use = use && fabsf(y[o]) <= tr.out_max;
         if (h.nD > T(0)) offered = 1.0f;
@@ -3466,7 +3473,8 @@ RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dy
       if (stage == 1) S.idm[c][i].w = mcrt;
       write_rec(P, S.rec, i, S.pos[c][i], S.vel[c][i], sg, S.idm[c][i].y, code.x >= 10);
     }
-    // statistics: one atomic per warp and counter
+    // statistics: kept per warp until the block ends (four atomics for
+    // every warp and tile queued at their one sector in L2)
     float so = offered, su = used, se = err, sx = err;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -3476,52 +3484,78 @@ RWD void closure_tile(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dy
       sx = fmaxf(sx, __shfl_xor_sync(0xffffffffu, sx, o));
     }
     if (lane == 0 && so > 0.0f) {
-      atomicAdd(&stats[0], (double)so);
-      atomicAdd(&stats[1], (double)su);
-      atomicAdd(&stats[2], (double)se);
-      atomicMax(reinterpret_cast<unsigned long long*>(&stats[3]), (unsigned long long)__double_as_longlong((double)sx));
+      stats[0] += (double)so;
+      stats[1] += (double)su;
+      stats[2] += (double)se;
+      stats[3] = fmax(stats[3], (double)sx);
     }
   }
 }
 
 // One integrator stage (0: predictor, 1: corrector) with the learned closure, in one
 // persistent launch: the rows of a tile are advanced as predictor_row / corrector_row do
-// (HypoCS stresses left to the closure), then the same block runs the closure on them.
+// (HypoCS stresses left to the closure), then the same 128 threads run the closure on them.
 // Tiles: the boundary rows first (integrator only), then the soil slots (in the predictor
 // the deleted slots too, for their step-start copies).
+// A tile is a chain of latencies (the rows' reads, ten barriers, five rounds of MMA, TMEM
+// read and tanh), so the SM needs many: two groups of 128 threads share a block's 29 KB of
+// weights and three blocks fit an SM in FP32 (80 registers, about 100 spilled bytes), 24 warps
+// instead of 16.  At 223k soil particles 86 us before, 63 now: the statistics' atomics, kept
+// per block now, cost 12, the third block 7, the second evaluation of the two powers 3 (four
+// blocks of one tile: 70; keeping all of HypoPre across the network spills 700 bytes: 70).
+// An FP64 row needs 168 registers: one tile a block, as many blocks as fit.
+template <class T> constexpr int kClGroups = sizeof(T) == 4 ? 2 : 1;  // tiles a block has at a time
+template <class T> constexpr int kClBlocks = sizeof(T) == 4 ? 3 : 4;  // blocks launched per SM
 template <class T, int Stage>
-__global__ void __launch_bounds__(mlp::TILE) k_integrate_cl(const Params<T> P, DevState<T> S, Dyn<T>* dyn,
-                                                             mlp::Net net, ClosureTrust tr, double* stats) {
+__global__ void __launch_bounds__(mlp::TILE * kClGroups<T>, sizeof(T) == 4 ? kClBlocks<T> : 1)
+    k_integrate_cl(const Params<T> P, DevState<T> S, Dyn<T>* dyn, mlp::Net net, ClosureTrust tr, double* stats) {
+  constexpr int kG = kClGroups<T>;
   extern __shared__ __align__(128) unsigned char raw[];
-  mlp::FwdSmem& sm = *reinterpret_cast<mlp::FwdSmem*>(raw);
-  mlp::load_fwd(sm, net);
-  if (threadIdx.x == 0) sm.err = 0;
-  mlp::block_setup(&sm.bar, &sm.tmem, 64);
+  mlp::FwdSmem<kG>& sm = *reinterpret_cast<mlp::FwdSmem<kG>*>(raw);
+  const int g = threadIdx.x / mlp::TILE, row = threadIdx.x & (mlp::TILE - 1);
+  mlp::FwdTile& ft = sm.t[g];
+  mlp::load_fwd(sm.w, net);
+  __shared__ double warp_stats[4 * kG][4];
+  double* const ws = warp_stats[threadIdx.x >> 5];
+  if ((threadIdx.x & 31) < 4) ws[threadIdx.x & 31] = 0.0;
+  if (row == 0) ft.err = 0;
+  if (threadIdx.x == 0)
+    for (int k = 1; k < kG; ++k) tc::mbar_init(&sm.t[k].bar, 1);
+  mlp::block_setup(&sm.t[0].bar, &sm.w.tmem, mlp::HID * kG);
   const int nb_tiles = (P.npb + mlp::TILE - 1) / mlp::TILE;
   const int soil_rows = Stage == 0 ? P.np - P.npb : dyn->npm;
   const int n_tiles = nb_tiles + (soil_rows + mlp::TILE - 1) / mlp::TILE;
   uint32_t phase = 0;
   const RowIn<T> in = row_in<T, Stage>(S, dyn);
-  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {  // block-uniform
+  for (int tile = blockIdx.x * kG + g; tile < n_tiles; tile += gridDim.x * kG) {  // group-uniform
     if (tile < nb_tiles) {
-      const int i = tile * mlp::TILE + threadIdx.x;
+      const int i = tile * mlp::TILE + row;
       if (i < P.npb) {
         if (Stage == 0) predictor_row<false>(P, S, dyn, i, in, i);
         else corrector_row(P, S, dyn, i, in, i);
       }
       continue;
     }
-    const int st = tile - nb_tiles, t = st * mlp::TILE + threadIdx.x;
+    const int st = tile - nb_tiles, t = st * mlp::TILE + row;
     if (t < soil_rows) {
       if (Stage == 0) predictor_row<false>(P, S, dyn, P.npb + t, in, P.npb + t);
       else corrector_row(P, S, dyn, P.npb + t, in, P.npb + t);
     }
-    closure_tile(P, S, dyn, sm, tr, stats, Stage, st, phase);
+    closure_tile(P, S, dyn, sm.w, ft, g, tr, ws, Stage, st, phase);
   }
-  __syncthreads();
-  mlp::drain_after_timeout(&sm.bar, sm.err, phase);
-  mlp::block_teardown(sm.tmem, 64);
-  if (threadIdx.x == 0 && sm.err) atomicOr(&dyn->err, 16u);
+  mlp::group_sync(g);
+  if (row == 0 && ft.err && phase > 0) tc::mbar_wait(&ft.bar, (phase - 1u) & 1u);  // MMAs of a late phase
+  mlp::block_teardown(sm.w.tmem, mlp::HID * kG);
+  if (threadIdx.x < 4) {  // after the barrier of the tear-down
+    double v = 0.0;
+    for (int k = 0; k < 4 * kG; ++k)
+      v = threadIdx.x < 3 ? v + warp_stats[k][threadIdx.x] : fmax(v, warp_stats[k][3]);
+    if (v != 0.0) {
+      if (threadIdx.x < 3) atomicAdd(&stats[threadIdx.x], v);
+      else atomicMax(reinterpret_cast<unsigned long long*>(&stats[3]), (unsigned long long)__double_as_longlong(v));
+    }
+  }
+  if (row == 0 && ft.err) atomicOr(&dyn->err, 16u);
 }
 
 }  // namespace rw

@@ -98,27 +98,28 @@ __device__ __forceinline__ int shuffled(long long s, long long n, long long a, l
 __global__ void __launch_bounds__(TILE) k_forward(Net net, const float* __restrict__ X, int n, float* __restrict__ Y,
                                                   int* err) {
   extern __shared__ __align__(128) unsigned char raw[];
-  FwdSmem& sm = *reinterpret_cast<FwdSmem*>(raw);
-  load_fwd(sm, net);
-  if (threadIdx.x == 0) sm.err = 0;
-  block_setup(&sm.bar, &sm.tmem, 64);
+  FwdSmem<1>& sm = *reinterpret_cast<FwdSmem<1>*>(raw);
+  FwdTile& t = sm.t[0];
+  load_fwd(sm.w, net);
+  if (threadIdx.x == 0) t.err = 0;
+  block_setup(&t.bar, &sm.w.tmem, 64);
   uint32_t phase = 0;
   for (int tile = blockIdx.x; tile * TILE < n; tile += gridDim.x) {
     const int s = tile * TILE + threadIdx.x;
     float f[IN];
 #pragma unroll
     for (int k = 0; k < IN; ++k) f[k] = s < n ? X[(size_t)s * IN + k] : 0.0f;
-    store_row<IN>(sm.x, threadIdx.x, f);
+    store_row<IN>(t.h, threadIdx.x, f);
     float out[OUT];
-    forward_tile(sm, 0, phase, out);
+    forward_tile(sm.w, t, 0, phase, out);
     if (s < n)
 #pragma unroll
       for (int o = 0; o < OUT; ++o) Y[(size_t)s * OUT + o] = out[o];
   }
   __syncthreads();
-  drain_after_timeout(&sm.bar, sm.err, phase);
-  block_teardown(sm.tmem, 64);
-  if (threadIdx.x == 0 && sm.err) atomicExch(err, 1);
+  drain_after_timeout(&t.bar, t.err, phase);
+  block_teardown(sm.w.tmem, 64);
+  if (threadIdx.x == 0 && t.err) atomicExch(err, 1);
 }
 
 // ---------------------------------------------------------------------------------
@@ -494,7 +495,7 @@ int num_sms(int dev) {
 // Forward of n samples already on the device.
 rw_status forward_dev(rw_mlp* m, const float* dx, int n, float* dy) {
   if (n <= 0) return RW_OK;
-  const int smem = (int)sizeof(FwdSmem);
+  const int smem = (int)sizeof(FwdSmem<1>);
   MLP_CU(m, cudaFuncSetAttribute(k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int tiles = (n + TILE - 1) / TILE;
   const int grid = std::min(tiles, 4 * num_sms(m->device));

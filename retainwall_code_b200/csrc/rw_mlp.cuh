@@ -102,23 +102,56 @@ __device__ __forceinline__ float load_elem(const unsigned char* tile, int r, int
   return __uint_as_float((uint32_t)u << 16);
 }
 
-// Shared memory of the forward pass of one 128-sample tile.
-struct FwdSmem {
+// Shared memory of a block's forward passes: the weights, and one tile's rows per group of 128
+// threads (the input rows lie where the hidden rows go: a layer's MMAs are done with theirs
+// before the next rows are written).  The hidden layers' biases are halved (silu_half).
+struct FwdWeights {
   alignas(128) unsigned char fw[FWBYTES];
-  alignas(128) unsigned char x[TILE * IN * 2];
-  alignas(128) unsigned char h[TILE * HID * 2];
-  float bias[NBIAS];
-  uint64_t bar;
+  alignas(16) float bias[NBIAS];
   uint32_t tmem;
-  int err;
+};
+struct FwdTile {
+  alignas(128) unsigned char h[TILE * HID * 2];
+  uint64_t bar;
+  int err, any;
+};
+template <int Groups> struct FwdSmem {
+  FwdWeights w;
+  FwdTile t[Groups];
 };
 
 // Copies the packed forward weights and biases into shared memory (all threads).
-__device__ __forceinline__ void load_fwd(FwdSmem& sm, const Net& net) {
+__device__ __forceinline__ void load_fwd(FwdWeights& w, const Net& net) {
   const uint4* src = reinterpret_cast<const uint4*>(net.fw);
-  uint4* dst = reinterpret_cast<uint4*>(sm.fw);
+  uint4* dst = reinterpret_cast<uint4*>(w.fw);
   for (int k = threadIdx.x; k < FWBYTES / 16; k += blockDim.x) dst[k] = src[k];
-  for (int k = threadIdx.x; k < NBIAS; k += blockDim.x) sm.bias[k] = net.bias[k];
+  for (int k = threadIdx.x; k < NBIAS; k += blockDim.x) w.bias[k] = net.bias[k] * (k < NHID * HID ? 0.5f : 1.0f);
+}
+
+// silu(v0 + b0), silu(v1 + b1) from the values and half the biases: z sigm(z) = h tanh(h) + h
+// with h = z / 2, two at a time in packed FP32 (two instructions, two tanh and a pack where
+// the scalar form took ten, two and a pack).
+__device__ __forceinline__ uint32_t silu_half2(float v0, float v1, float2 hb) {
+  unsigned long long z, t, half, b;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(z) : "f"(v0), "f"(v1));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(half) : "f"(0.5f));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(hb.x), "f"(hb.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(z) : "l"(z), "l"(half), "l"(b));
+  float h0, h1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(h0), "=f"(h1) : "l"(z));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "f"(tc::tanh_approx(h0)), "f"(tc::tanh_approx(h1)));
+  asm("fma.rn.f32x2 %0, %1, %2, %1;" : "=l"(z) : "l"(z), "l"(t));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(h0), "=f"(h1) : "l"(z));
+  return pack_bf16(h0, h1);
+}
+
+// Barriers of one group's 128 threads, group 0..3 (named by constants: with a number in a
+// register the block would claim all sixteen).
+__device__ __forceinline__ void group_sync(int g) {
+  if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+  else if (g == 1) asm volatile("bar.sync 2, 128;" ::: "memory");
+  else if (g == 2) asm volatile("bar.sync 3, 128;" ::: "memory");
+  else asm volatile("bar.sync 4, 128;" ::: "memory");
 }
 
 // Issues the MMAs of layer l (0..4) of one tile: A = x (l = 0) or h, B = packed W^T,
@@ -133,46 +166,53 @@ __device__ __forceinline__ void issue_layer(const unsigned char* a_tile, int K, 
                  ks > 0 ? 1u : 0u);
 }
 
-// Forward pass of the tile already in sm.x (rows = threads of this 128-thread block).
-// TMEM: columns [tcol, tcol + 64) of the allocation at sm.tmem.  Each thread receives
-// its row's six outputs (biases added).  phase counts the mbarrier phases used so far.
-// A wait that times out sets sm.err: the outputs are then meaningless, and this and
-// every later call issue no further MMAs (all threads see sm.err after the barrier at
-// the top of a layer and return together).
-__device__ __forceinline__ void forward_tile(FwdSmem& sm, int tcol, uint32_t& phase, float* out) {
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t tbase = sm.tmem + (uint32_t)tcol;
-  const uint32_t tlane = tbase + ((uint32_t)(warp * 32) << 16);
+// Forward pass of the tile whose input rows are in t.h (stored as IN columns; row = thread of
+// the group, g the group's number).  TMEM: columns [64 g, 64 g + 64) of the allocation at
+// w.tmem.  Each thread receives its row's six outputs (biases added).  phase counts the
+// mbarrier phases used so far.  A wait that times out sets t.err: the outputs are then
+// meaningless, and this and every later call issue no further MMAs (the group's threads see
+// t.err after the barrier at the top of a layer and return together).
+__device__ __forceinline__ void forward_tile(const FwdWeights& w, FwdTile& t, int g, uint32_t& phase, float* out) {
+  const int row = threadIdx.x & (TILE - 1);
+  const uint32_t tbase = w.tmem + 64u * (uint32_t)g;
+  const uint32_t tlane = tbase + ((uint32_t)(row & ~31) << 16);
+#pragma unroll 1
   for (int l = 0; l <= NHID; ++l) {
     tc::fence_smem_to_async();
-    __syncthreads();
-    if (sm.err) return;
-    if (tid == 0) {
+    group_sync(g);
+    if (t.err) return;
+    if (row == 0) {
       tc::fence_after_sync();
-      if (l == 0) issue_layer(sm.x, IN, sm.fw + FW1, HID, tbase);
-      else if (l < NHID) issue_layer(sm.h, HID, sm.fw + (l == 1 ? FW2 : l == 2 ? FW3 : FW4), HID, tbase);
-      else issue_layer(sm.h, HID, sm.fw + FW5, OUTP, tbase);
-      tc::mma_commit(&sm.bar);
+      if (l == 0) issue_layer(t.h, IN, w.fw + FW1, HID, tbase);
+      else if (l < NHID) issue_layer(t.h, HID, w.fw + FW2 + (l - 1) * (FW3 - FW2), HID, tbase);
+      else issue_layer(t.h, HID, w.fw + FW5, OUTP, tbase);
+      tc::mma_commit(&t.bar);
     }
-    if (!tc::mbar_wait(&sm.bar, phase & 1u)) sm.err = 1;
+    if (!tc::mbar_wait(&t.bar, phase & 1u)) t.err = 1;
     ++phase;
     tc::fence_after_sync();
     if (l < NHID) {
-      const float* b = sm.bias + l * HID;
 #pragma unroll 1
-      for (int c = 0; c < HID; c += 16) {
-        float v[16];
-        tc::tmem_ld16(tlane + (uint32_t)c, v);
+      for (int c = 0; c < HID; c += 32) {
+        const float2* b = reinterpret_cast<const float2*>(w.bias + l * HID + c);
+        float v[32];
+        tc::tmem_ld32(tlane + (uint32_t)c, v);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = silu(v[k] + b[c + k]);
-        store_chunk16<HID>(sm.h, tid, c, v);
+        for (int k = 0; k < 32; k += 8) {
+          uint4 q;
+          q.x = silu_half2(v[k], v[k + 1], b[k / 2]);
+          q.y = silu_half2(v[k + 2], v[k + 3], b[k / 2 + 1]);
+          q.z = silu_half2(v[k + 4], v[k + 5], b[k / 2 + 2]);
+          q.w = silu_half2(v[k + 6], v[k + 7], b[k / 2 + 3]);
+          *reinterpret_cast<uint4*>(t.h + tc::kmajor_off(row, c + k, HID)) = q;
+        }
       }
       tc::fence_before_sync();
     } else {
       float v[16];
       tc::tmem_ld16(tlane, v);
 #pragma unroll
-      for (int o = 0; o < OUT; ++o) out[o] = v[o] + sm.bias[NHID * HID + o];
+      for (int o = 0; o < OUT; ++o) out[o] = v[o] + w.bias[NHID * HID + o];
       tc::fence_before_sync();
     }
   }
