@@ -47,17 +47,17 @@ def metric_of(workload: str) -> str:
     """The headline metric for the 1.92M wall; the same quantity named for the other cases."""
     return METRICS.get(workload, METRIC)
 # From the ncu capture of the interaction's walk kernel on the 0.96M-particle case
-# (profiles/k_interaction_wall2_half.md): DRAM read+write 461.4 + 63.4 MB and 337.2M warp
+# (profiles/k_interaction_wall2_half.md): DRAM read+write 461.4 + 63.4 MB and 260M warp
 # instructions per launch.  Both grow with the particle count, so they are scaled per
 # soil particle to the benchmarked case.
 IX_DRAM_BYTES_PER_SOIL = (461.41e6 + 63.44e6) / 960000
-IX_WARP_INSTR_PER_SOIL = 337.22e6 / 960000
+IX_WARP_INSTR_PER_SOIL = 260e6 / 960000
 # L1 data-stage wavefronts the walk kernel cannot avoid: each listed neighbour's 64-byte
 # record is two 32-byte sectors read by one lane (records of a warp's lanes are distinct),
 # each list entry an eighth of a sector (a warp's 32 entries are one coalesced 128-byte
-# load), each particle's own state and outputs about 240 B.  The L1 data stage retires one
-# wavefront per cycle per SM, and scattered sectors cost one wavefront each (ncu: 122.5M
-# sectors requested per launch on the 0.96M case, 84% of the stage's peak).
+# load), each particle's own state and outputs about 240 B.  The L1 data stage serves two
+# scattered sectors per cycle per SM where they lie in different halves of a 64-byte
+# record, as odd and even lanes read them; a sector that is not in L1 costs a cycle more.
 IX_L1_SECTORS_PER_ENTRY = 2 + 1 / 8
 IX_L1_SECTORS_PER_SOIL = 240 / 32
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
@@ -590,11 +590,12 @@ def run_ours(args, ws, rank, local):
              "unit": "warp-instructions/s", "frac": issue_ach / issue_peak,
              "note": "instructions per launch from the ncu capture, scaled per soil particle"}
     l1_sectors = IX_L1_SECTORS_PER_ENTRY * list_entries + IX_L1_SECTORS_PER_SOIL * npm
-    l1_peak = 148 * mhz * 1e6  # one L1 data-stage wavefront per cycle per SM
+    l1_peak = 2 * 148 * mhz * 1e6  # two scattered sectors per cycle per SM
     roof_l1 = {"bound": "L1 data stage", "kernel": "k_interaction", "achieved": l1_sectors / (ix_ms * 1e-3),
                "peak": l1_peak, "unit": "sectors/s", "frac": l1_sectors / (ix_ms * 1e-3) / l1_peak,
                "sectors_per_launch": l1_sectors,
-               "note": "2 sectors per listed neighbour (64-B record) + 1/8 per list entry + 7.5 per particle"}
+               "note": "2 sectors per listed neighbour (64-B record) + 1/8 per list entry + 7.5 per particle; "
+                       "sectors that miss L1 (about a quarter) cost a cycle more and are not counted"}
     line = {
         "metric": metric_of(args.workload), "value": value, "unit": "particle-updates/s", "n_gpus": ws,
         "steps": args.steps,

@@ -124,11 +124,12 @@ typedef struct rw_info {
   double time, dt, h, dr;
   int32_t n_sorts;       /* neighbour-search sections whose sort permuted the particles     */
   int32_t n_list_reuse;  /* interactions that walked kept candidate lists                    */
-  int32_t n_search_skipped; /* captured-step searches skipped whole (no particle changed cell)  */
+  int32_t n_search_skipped; /* gated searches (captured steps, and stage calls from a context's
+                               third step on) skipped whole (no particle changed cell)          */
   int32_t n_scan_skipped;   /* captured-step interactions whose scan launch was skipped (every
                                particle walked a kept list)                                      */
-  int32_t n_build_skipped;     /* captured-step interactions whose list build was skipped (the
-                                  kept lists stood)                                              */
+  int32_t n_build_skipped;     /* gated searches whose list build was skipped (the kept lists
+                                  stood)                                                         */
   int32_t graph_kernels;       /* kernels of one captured step when no gated body is skipped     */
   int32_t search_body_kernels; /* kernels a skipped search does not launch                       */
   int32_t n_list_updates;      /* interactions that updated the kept lists in part: rebuilt those
@@ -170,11 +171,12 @@ enum {
                                    may have moved 0.45 skin since the last full build.  Results do not
                                    depend on it. */
   RW_OPT_GRAPH_GATES = 6,       /* 1 (default): the captured step graph skips a search with no cell change
-                                   and an idle scan launch behind conditional nodes; 0: plain graph, every
-                                   kernel launched (profilers that replay single graph kernels need it).
+                                   and an idle scan launch behind conditional nodes, and the search of a
+                                   stage call does so in a graph of its own; 0: plain graph, every kernel
+                                   launched (profilers that replay single graph kernels need it).
                                    Results do not depend on it. */
-  RW_OPT_WALK_THREADS = 8,      /* threads per block of the interaction's walk launch: 64 or 128 (default);
-                                   results do not depend on it */
+  RW_OPT_WALK_THREADS = 8,      /* threads per block of the interaction's walk launch: 64 or 128 (default;
+                                   at most two such blocks per SM take 64); results do not depend on it */
   RW_OPT_INTEGRATOR_THREADS = 9, /* threads per block of the predictor and corrector: 128 or 256 (default);
                                    results do not depend on it */
   RW_OPT_CLOSURE_MAX_ERR = 7,   /* learned closure: a particle keeps the network's objective rate only while
