@@ -906,12 +906,11 @@ template <class T>
 RWD void adami_finish(const Params<T>& P, const DevState<T>& S, const Dyn<T>* dyn, int c, int i, bool contact,
                       const int4& code, const V3<T> pos_i, const I3 celli, const V3<T> n_i, const S6<T>& rs,
                       const V4<T>& rps, const V4<T>& rvr) {
-  const V4<T>* __restrict__ vel = S.vel[c];
   const T nn = f_sqrt(f_fma(n_i.z, n_i.z, f_fma(n_i.y, n_i.y, rmul(n_i.x, n_i.x))));
   if (nn > T(0)) {
     S.cny[i] = V4<T>{n_i.x / nn, n_i.y / nn, n_i.z / nn, T(0)};
   }
-  V4<T> vr_out = vel[i];
+  V4<T> vr_out = S.vel[c][i];
   S6<T> str_out;
   if (rps.w > T(0.0f)) {
     const T kersum = rps.w;
@@ -1058,12 +1057,14 @@ template <class T> __global__ void __launch_bounds__(128) k_adami(const Params<T
       S6<T> sj[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        // no particle: the boundary particle itself, its term not added below
-        const int j = (ent[k] & kNone) == kNone ? i : (int)(ent[k] & kNone);
+        // no particle: the boundary particle itself, its term not added below.  Only the
+        // position of a boundary neighbour counts; velocity and stress of boundary rows are
+        // written by this launch, so those lanes read the first soil row instead
+        const int j = (ent[k] & kNone) == kNone ? i : (int)(ent[k] & kNone), m = max(j, P.npb);
         pj[k] = pos[j];
-        vj[k] = vel[j];
-        mj[k] = idm[j].y;
-        sj[k] = ld6(sa, sb, j);
+        vj[k] = vel[m];
+        mj[k] = idm[m].y;
+        sj[k] = ld6(sa, sb, m);
       }
       entries(e0 + 4, nxt);
       // The four kernels and volumes are formed side by side without a branch (square
@@ -1143,9 +1144,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_adami_group(const Params<T> P
   unsigned ent = group_entry(nbb, (size_t)P.npb, i, e, cnt, own);
   for (int r = 0; r < rounds; ++r, e += kLanes, buf ^= 1) {
     const int j = (int)(ent & kEntIdx);
-    const V4<T> pj = pos[j], vj = vel[j];
-    const T mj = idm[j].y;
-    const S6<T> sj = ld6(sa, sb, j);
+    const int m = max(j, P.npb);  // boundary rows are written by this launch (see k_adami)
+    const V4<T> pj = pos[j], vj = vel[m];
+    const T mj = idm[m].y;
+    const S6<T> sj = ld6(sa, sb, m);
     const V3<T> off = mulI(entry_off(ent), th);
     const bool valid = e < cnt, wall = j < P.npb;
     ent = group_entry(nbb, (size_t)P.npb, i, e + kLanes, cnt, own);
