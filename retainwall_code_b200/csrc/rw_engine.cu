@@ -544,6 +544,13 @@ template <class T> struct Engine final : EngineBase {
   bool search_graph(int section) {
     if (gsearch[section]) return true;
     if (gsearch_refused) return false;
+    // Instantiation allocates, which would void a capture that the caller has open on another
+    // stream (global mode); nothing made here can become part of that capture.
+    struct Relaxed {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+      ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    } relaxed;
     cudaGraph_t g = nullptr;
     RW_CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     allow_cond = true;
