@@ -98,7 +98,7 @@ template <class T> struct Engine final : EngineBase {
   cudaGraphExec_t gexec = nullptr;
   cudaGraphExec_t gsearch[2] = {nullptr, nullptr};  // neighbor_search of a stage call, by section
   bool gsearch_refused = false;
-  int stage_searches = 0;
+  int stage_searches = 0, search_wait = 4;  // searches of stage calls since an option changed; those without a graph
   int g_cpar = -1;
   int ix_kernel = 0;     // 0: neighbours through L1/L2 (default); 1: chunked, shared-memory position tile
   int walk_threads = 128;   // RW_OPT_WALK_THREADS: block size of the walk launch
@@ -530,7 +530,7 @@ template <class T> struct Engine final : EngineBase {
   void neighbor_search(int section) override {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RW_CU(cudaStreamIsCapturing(st, &cs));
-    if (cs == cudaStreamCaptureStatusNone && graph_gates && ++stage_searches > 4 && search_graph(section)) {
+    if (cs == cudaStreamCaptureStatusNone && graph_gates && ++stage_searches > search_wait && search_graph(section)) {
       RW_CU(cudaGraphLaunch(gsearch[section], st));
       return;
     }
@@ -539,8 +539,10 @@ template <class T> struct Engine final : EngineBase {
   // The search of a stage call as a graph of its own, behind the same gates as in the step
   // graph: most searches have nothing to do, and their 17 launches that return at once cost
   // more than a small case's kernels (56k-particle wall, stage calls: 0.37 ms a step, 0.27
-  // this way).  Made once a host program has called the stages for two steps (0.15 ms each).
-  // False: conditional nodes refused, launched plainly.
+  // this way).  Made (0.15 ms each) once a host program has called the stages for two steps
+  // with its options unchanged; whenever an option drops graphs that had been made, twice as
+  // many searches go by before the next ones, so a program that keeps setting options ends up
+  // with plain launches.  False: conditional nodes refused, launched plainly.
   bool search_graph(int section) {
     if (gsearch[section]) return true;
     if (gsearch_refused) return false;
@@ -574,6 +576,8 @@ template <class T> struct Engine final : EngineBase {
   }
   // Captured launches hold the parameters and options of their capture.
   void drop_graphs() {
+    if (gsearch[0] || gsearch[1]) search_wait = std::min(2 * search_wait, 1 << 20);
+    stage_searches = 0;
     for (cudaGraphExec_t* g : {&gexec, &gsearch[0], &gsearch[1]})
       if (*g) {
         cudaGraphExecDestroy(*g);
