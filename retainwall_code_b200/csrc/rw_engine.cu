@@ -553,20 +553,13 @@ template <class T> struct Engine final : EngineBase {
       Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
       ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
     } relaxed;
-    cudaGraph_t g = nullptr;
-    RW_CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    allow_cond = true;
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = cudaErrorNotSupported;
     try {
-      launch_search(section);
+      cudaGraph_t g = capture(true, [&] { launch_search(section); });
+      e = cudaGraphInstantiate(&gsearch[section], g, 0);
+      cudaGraphDestroy(g);
     } catch (const Fail&) {
-      e = cudaErrorNotSupported;
     }
-    allow_cond = false;
-    const cudaError_t ended = cudaStreamEndCapture(st, &g);
-    if (e == cudaSuccess) e = ended;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&gsearch[section], g, 0);
-    if (g) cudaGraphDestroy(g);
     if (e != cudaSuccess) {
       cudaGetLastError();
       gsearch[section] = nullptr;
@@ -858,22 +851,28 @@ template <class T> struct Engine final : EngineBase {
   // cond: gate the search, the list build and the scan launch with conditional nodes
   // (gated()).  The batch's fallback nests step graphs as child graphs, without.
   cudaGraph_t capture_step(bool cond = false) {
-    cudaGraph_t g = nullptr;
     const int c0 = cpar;
+    struct Restore {  // the step runs two interactions: parity is back where it started
+      int &now, was;
+      ~Restore() { now = was; }
+    } restore{cpar, c0};
+    return capture(cond, [&] { launch_step(); });
+  }
+  // What body launches, as a graph; the capture is ended whatever body throws.
+  template <class F> cudaGraph_t capture(bool cond, F&& body) {
+    cudaGraph_t g = nullptr;
     RW_CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     allow_cond = cond;
     try {
-      launch_step();
+      body();
     } catch (...) {
       allow_cond = false;
       cudaStreamEndCapture(st, &g);
       if (g) cudaGraphDestroy(g);
-      cpar = c0;
       throw;
     }
     allow_cond = false;
     RW_CU(cudaStreamEndCapture(st, &g));
-    cpar = c0;  // the step runs two interactions: parity is back where it started
     return g;
   }
 
