@@ -175,8 +175,9 @@ enum {
                                    stage call does so in a graph of its own; 0: plain graph, every kernel
                                    launched (profilers that replay single graph kernels need it).
                                    Results do not depend on it. */
-  RW_OPT_WALK_THREADS = 8,      /* threads per block of the interaction's walk launch: 64 or 128 (default;
-                                   at most two such blocks per SM take 64); results do not depend on it */
+  RW_OPT_WALK_THREADS = 8,      /* threads per block of the interaction's walk launch: 64 or 128; without it
+                                   128, and 64 in small FP64 cases (rw_info.walk_threads says which);
+                                   results do not depend on it */
   RW_OPT_INTEGRATOR_THREADS = 9, /* threads per block of the predictor and corrector: 128 or 256 (default);
                                    results do not depend on it */
   RW_OPT_CLOSURE_MAX_ERR = 7,   /* learned closure: a particle keeps the network's objective rate only while

@@ -101,7 +101,7 @@ template <class T> struct Engine final : EngineBase {
   int stage_searches = 0, search_wait = 4;  // searches of stage calls since an option changed; those without a graph
   int g_cpar = -1;
   int ix_kernel = 0;     // 0: neighbours through L1/L2 (default); 1: chunked, shared-memory position tile
-  int walk_threads = 128;   // RW_OPT_WALK_THREADS: block size of the walk launch
+  int walk_threads = 0;     // RW_OPT_WALK_THREADS: block size of the walk launch (0: not set, walk_block decides)
   int integ_threads = 256;  // RW_OPT_INTEGRATOR_THREADS: block size of the predictor and corrector
   bool strict_fp = false;  // interaction arithmetic: fused multiply-adds (default) or separately rounded
   int ncol = 0, max_chunks = 0;
@@ -599,6 +599,17 @@ template <class T> struct Engine final : EngineBase {
     // the second pass over a periodic image runs on one lane of the eight
     return !P.periodbound && std::max(beside_soil, (long)(P.np - P.npb)) <= (sizeof(T) == 4 ? 16384 : 12288);
   }
+  // Block size of the walk launch: the caller's, or else 128 threads, and 64 in FP64 where
+  // blocks of 128 are at most two per SM and a thread takes a particle: few blocks fill the
+  // SMs unevenly (27,648 particles are 216 blocks of 128 on 148 SMs).  us a launch, blocks of
+  // 64 / 128: FP64 57 / 61 at 20.8k, 59 / 66 at 27.6k, 69 / 68 at 33.8k, 66 / 69 at 37.9k;
+  // FP32 34 / 33, 36 / 34, 38 / 38, 36 / 38.  Eight lanes per particle share rows of a fixed
+  // size, so blocks of 64 hold fewer warps: FP64 42 / 32 at 6.8k, FP32 30 / 28 at 13.7k.
+  int walk_block() const {
+    if (walk_threads) return walk_threads;
+    const bool lanes = !strict_fp && lists_kept() && walk_lanes();
+    return sizeof(T) == 8 && !lanes && nblk(P.np - P.npb, 128) <= 2 * (unsigned)nsm ? 64 : 128;
+  }
   bool adami_lanes() const {
     return lists_kept() && S.nbb[0] && std::max(beside_bnd, (long)P.npb) <= (sizeof(T) == 4 ? 40960 : 16384);
   }
@@ -689,9 +700,7 @@ template <class T> struct Engine final : EngineBase {
                 if (strict_fp) k_interaction<T, true, false><<<g, IX_THREADS, sm1, st>>>(P, S, d_dyn, cpar);
                 else k_interaction<T, false, false><<<g, IX_THREADS, sm1, st>>>(P, S, d_dyn, cpar);
               });
-        // At most two blocks of 128 per SM: blocks of 64 fill the SMs more evenly (27,648
-        // particles are 216 blocks on 148 SMs; FP64 walk 66 -> 59 us, FP32 the same).
-        const int wt = nblk(n, 128) <= 2 * (unsigned)nsm ? std::min(walk_threads, 64) : walk_threads;
+        const int wt = walk_block();
         const unsigned gw = nblk(n, wt);
         if (!strict_fp && lists_kept() && walk_lanes())
           k_interaction_group<T><<<nblk((long)n * kLanes, wt), wt, 0, st>>>(P, S, d_dyn, cpar);
@@ -1071,7 +1080,7 @@ template <class T> struct Engine final : EngineBase {
     o->time_max = cparams.time_max;
     o->output_frequency = cparams.output_frequency;
     o->ix_kernel = ix_kernel;
-    o->walk_threads = walk_threads;
+    o->walk_threads = walk_block();
     o->integrator_threads = integ_threads;
   }
 
