@@ -4,6 +4,7 @@
 // deleted cell), so the 27 neighbour cells of a particle are 9 contiguous index runs
 // per layer and neighbour reads of consecutive particles hit the same lines.
 #pragma once
+#include <float.h>
 #include <limits.h>
 
 #include "rw_device.cuh"
@@ -1673,6 +1674,12 @@ RWD float div_ftz(float a, float b) {
   asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
   return y;
 }
+// f_fastdiv(a, b) for a quotient that is nearly always negative and normal: the flushing form
+// then gives the same value; anything else is divided again.
+RWD float div_negative(float a, float b) {
+  const float y = div_ftz(a, b);
+  return y <= -FLT_MIN && y >= -FLT_MAX ? y : f_fastdiv(a, b);
+}
 
 // gv -= a (x) b where ok holds.
 RWD void add_grad(Acc<float>& A, float ax, float ay, float az, float bx, float by, float bz, bool ok) {
@@ -1815,8 +1822,8 @@ RWD void ix_walk_pairs(const Params<float>& P, const DevState<float>& S, const I
     const F2 vd = dot2(wx, wy, wz, dx, dy, dz);
     const F2 num = mul2(f2(P.visc_k), vd);
     const F2 den = mul2(add2(r2, f2(P.eta)), mul2(f2(0.5f), add2(rho_i, rho_j)));
-    const F2 artv = f2(f2_lo(vd) < 0.0f ? div_ftz(f2_lo(num), f2_lo(den)) : 0.0f,
-                       f2_hi(vd) < 0.0f ? div_ftz(f2_hi(num), f2_hi(den)) : 0.0f);
+    const F2 artv = f2(f2_lo(vd) < 0.0f ? div_negative(f2_lo(num), f2_lo(den)) : 0.0f,
+                       f2_hi(vd) < 0.0f ? div_negative(f2_hi(num), f2_hi(den)) : 0.0f);
     const F2 mv = mul2(mass, artv);
     const F2 tr = add2(add2(jxx, jyy), jzz);
     // the sums of one pair, predicated instead of branched over (a lane or two of a warp
