@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/retainwall.h"
+#include "rw_host.h"
 #include "rw_io.h"
 #include "rw_kernels.cuh"
 
@@ -1180,27 +1181,6 @@ template <class T> struct Engine final : EngineBase {
     return P.np;
   }
 
-  // Writes to every page of a large destination from several host threads: the page faults
-  // of new memory otherwise run on the one thread that copies (a 35 MB array in 5 ms; 20 ms
-  // through a temporary vector on one thread).  Page-locked slots were slower to make (3 to
-  // 60 ms) than they saved.
-  static void touch(void* dst, size_t bytes) {
-    constexpr size_t kPage = 4096, kPerThread = 2u << 20;
-    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t of = std::min(bytes / kPerThread, std::min<size_t>(hw, 8));
-    auto part = [=](size_t w) {
-      volatile unsigned char* p = static_cast<unsigned char*>(dst);
-      for (size_t k = bytes * w / of; k < bytes * (w + 1) / of; k += kPage) p[k] = 0;
-    };
-    std::vector<std::thread> th;
-    try {
-      for (size_t w = 1; w < of; ++w) th.emplace_back(part, w);
-    } catch (const std::system_error&) {  // the copy meets the other pages itself
-    }
-    if (of) part(0);
-    for (auto& x : th) x.join();
-  }
-
   int get_array(int which, void* dst, size_t bytes) override {
     if (which < 0 || which >= RW_ARR_COUNT_) return RW_EINVAL;
     const size_t n = rows(which), rb = row_bytes(which);
@@ -1225,7 +1205,7 @@ template <class T> struct Engine final : EngineBase {
       }
     };
     auto put6 = [&](const V4<T>* a, const V2<T>* b) { put_rows(Rows6<T>{a, b}); };
-    touch(dst, bytes);
+    touch_pages(dst, bytes);
     switch (which) {
       case RW_ARR_CODES: put(S.codes[c]); break;
       case RW_ARR_CELLPOS: put(S.cellpos[c]); break;

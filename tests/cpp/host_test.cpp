@@ -1,0 +1,35 @@
+// Checks of csrc/rw_host.h, one per command-line argument; prints what failed.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+
+#include "rw_host.h"
+
+// A destination's contents survive, whatever its alignment and whether its pages are mapped.
+static bool contents() {
+  const size_t big = (size_t)40 << 20;
+  for (size_t bytes : {(size_t)0, (size_t)1, (size_t)4095, (size_t)3 << 20, big - 5})
+    for (size_t shift : {0, 1, 4093}) {
+      unsigned char* p = static_cast<unsigned char*>(std::malloc(big + 8192));
+      for (size_t k = 0; k < big + 8192; ++k) p[k] = (unsigned char)(k * 2654435761u >> 7);
+      rw::touch_pages(p + shift, bytes);
+      for (size_t k = 0; k < big + 8192; ++k)
+        if (p[k] != (unsigned char)(k * 2654435761u >> 7)) return false;
+      std::free(p);
+    }
+  unsigned char* z = static_cast<unsigned char*>(std::calloc(big, 1));  // not mapped yet
+  rw::touch_pages(z, big);
+  for (size_t k = 0; k < big; ++k)
+    if (z[k]) return false;
+  std::free(z);
+  return true;
+}
+
+int main(int argc, char** argv) {
+  const std::string which = argc > 1 ? argv[1] : "";
+  bool ok = false;
+  if (which == "contents") ok = contents();
+  if (!ok) std::printf("%s failed\n", which.c_str());
+  return ok ? 0 : 1;
+}
