@@ -2,9 +2,8 @@
 #pragma once
 #include <algorithm>
 #include <cstddef>
-#include <system_error>
+#include <exception>
 #include <thread>
-#include <vector>
 
 namespace rw {
 
@@ -15,20 +14,21 @@ namespace rw {
 // Page-locked slots were slower to make (3 to 60 ms) than they saved, and populating on
 // request (madvise) slower than the faults (122 MB in three arrays: 22 ms, 18 this way).
 inline void touch_pages(void* dst, size_t bytes) {
-  constexpr size_t kPage = 4096, kPerThread = 2u << 20;
+  constexpr size_t kPage = 4096, kPerThread = 2u << 20, kThreads = 8;
   const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t of = std::min(bytes / kPerThread, std::min<size_t>(hw, 8));
+  const size_t of = std::min(bytes / kPerThread, std::min(hw, kThreads));
   auto part = [=](size_t w) {
     unsigned char* p = static_cast<unsigned char*>(dst);
     for (size_t k = bytes * w / of; k < bytes * (w + 1) / of; k += kPage) __atomic_fetch_or(p + k, 0, __ATOMIC_SEQ_CST);
   };
-  std::vector<std::thread> th;
+  std::thread th[kThreads];  // an array: a vector that fails to grow would destroy running threads
+  size_t started = 1;
   try {
-    for (size_t w = 1; w < of; ++w) th.emplace_back(part, w);
-  } catch (const std::system_error&) {  // the copy meets the other pages itself
+    for (; started < of; ++started) th[started] = std::thread(part, started);
+  } catch (const std::exception&) {  // no thread or no memory: the copy meets the other pages itself
   }
   if (of) part(0);
-  for (auto& x : th) x.join();
+  for (size_t w = 1; w < started; ++w) th[w].join();
 }
 
 }  // namespace rw

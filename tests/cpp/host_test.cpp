@@ -1,10 +1,24 @@
 // Checks of csrc/rw_host.h, one per command-line argument; prints what failed.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
-#include <cstring>
+#include <new>
 #include <string>
 
 #include "rw_host.h"
+
+// Allocations left before operator new fails (negative: it does not).
+static std::atomic<int> g_left{-1};
+void* operator new(size_t n) {
+  if (g_left >= 0 && g_left.fetch_sub(1) <= 0) {
+    g_left = 0;
+    throw std::bad_alloc();
+  }
+  if (void* p = std::malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 // A destination's contents survive, whatever its alignment and whether its pages are mapped.
 static bool contents() {
@@ -26,10 +40,24 @@ static bool contents() {
   return true;
 }
 
+// Host memory that runs out at any allocation ends neither the call nor the process.
+static bool no_memory() {
+  const size_t big = (size_t)40 << 20;
+  unsigned char* p = static_cast<unsigned char*>(std::calloc(big, 1));
+  for (int left = 0; left < 20; ++left) {
+    g_left = left;
+    rw::touch_pages(p, big);
+    g_left = -1;
+  }
+  std::free(p);
+  return true;
+}
+
 int main(int argc, char** argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   bool ok = false;
   if (which == "contents") ok = contents();
+  if (which == "no_memory") ok = no_memory();
   if (!ok) std::printf("%s failed\n", which.c_str());
   return ok ? 0 : 1;
 }
