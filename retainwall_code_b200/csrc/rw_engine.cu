@@ -396,7 +396,7 @@ template <class T> struct Engine final : EngineBase {
       tab = dalloc<HypoC<T>>(kModelMax);
       d_clstats = dalloc<double>(4);
       d_count = dalloc<unsigned long long>(1);
-      export_bytes = std::min<size_t>(9 * sizeof(T) * np, 8u << 20);
+      export_bytes = export_buffer_bytes((size_t)np, (size_t)P.ncell, sizeof(T));
       d_export = dalloc<unsigned char>(export_bytes);
       d_dyn = dalloc<Dyn<T>>(1);
     };

@@ -31,4 +31,11 @@ inline void touch_pages(void* dst, size_t bytes) {
   for (size_t w = 1; w < started; ++w) th[w].join();
 }
 
+// Bytes of the device buffer that exports are put together in: the widest array per particle
+// (nine scalars) or the cells' begins whole, up to 8 MB (then in pieces of that; a piece costs
+// a launch and a copy, so a small case in a large grid is not cut by its particle count).
+inline size_t export_buffer_bytes(size_t np, size_t ncell, size_t scalar) {
+  return std::min<size_t>(std::max(9 * scalar * np, sizeof(int) * ncell), 8u << 20);
+}
+
 }  // namespace rw

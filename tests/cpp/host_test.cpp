@@ -53,11 +53,27 @@ static bool no_memory() {
   return true;
 }
 
+// Every array in the fewest pieces that 8 MB allow, also where cells outnumber particles.
+static bool export_pieces() {
+  for (size_t scalar : {4, 8})
+    for (size_t np : {1, 1000, 60000, 2180000})
+      for (size_t ncell : {1, 37404, 2000000, 30000000}) {
+        const size_t buf = rw::export_buffer_bytes(np, ncell, scalar);
+        if (buf > (8u << 20)) return false;
+        for (size_t bytes : {9 * scalar * np, 6 * scalar * np, 4 * ncell}) {
+          const size_t pieces = (bytes + buf - 1) / buf;
+          if (pieces > (bytes + (8u << 20) - 1) / (8u << 20)) return false;
+        }
+      }
+  return true;
+}
+
 int main(int argc, char** argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   bool ok = false;
   if (which == "contents") ok = contents();
   if (which == "no_memory") ok = no_memory();
+  if (which == "export_pieces") ok = export_pieces();
   if (!ok) std::printf("%s failed\n", which.c_str());
   return ok ? 0 : 1;
 }

@@ -15,7 +15,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["contents", "no_memory"])
+@pytest.mark.parametrize("check", ["contents", "no_memory", "export_pieces"])
 def test_host_helper(program, check):
     r = subprocess.run([program, check], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
