@@ -442,11 +442,15 @@ struct rw_mlp {
   float* stg = nullptr;
   long long cap = 0, n = 0;
   // Device copy of the host arrays of rw_mlp_forward / rw_mlp_grad, kept between calls up to
-  // kKeep bytes (a stream-ordered allocation goes back to the driver at each wait: 0.2 to
-  // 2 ms a call), larger ones allocated for the call.
-  static constexpr size_t kKeep = 64u << 20;
+  // kKeep bytes; more is allocated for the call, in stream order (given back to the driver at
+  // the wait: 0.2 to 2 ms a call, which is why smaller ones are kept).  Sizes are kFirst times a
+  // power of two, and outgrown buffers stay until the network goes: cudaFree waits for the work
+  // of every stream on the device.
+  static constexpr size_t kKeep = 64u << 20, kFirst = 1u << 20;
   unsigned char* ws = nullptr;
   size_t ws_bytes = 0;
+  void* outgrown[8] = {};
+  int n_outgrown = 0;
   std::string msg;
   std::mutex mu;
 };
@@ -531,26 +535,28 @@ struct CallBuffer {
       return RW_OK;
     }
     own = bytes > rw_mlp::kKeep;
-    if (!own && m->ws) {  // the last call's work was waited for
-      cudaFree(m->ws);
-      m->ws = nullptr;
-      m->ws_bytes = 0;
+    if (!own) {
+      size_t size = rw_mlp::kFirst;
+      while (size < bytes) size *= 2;
+      bytes = size;
     }
-    const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+    const cudaError_t e = own ? cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, m->st)
+                              : cudaMalloc(reinterpret_cast<void**>(&p), bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
       return fail(m, RW_ECUDA, std::string("device memory of the call: ") + cudaGetErrorString(e));
     }
     if (!own) {
+      if (m->ws) m->outgrown[m->n_outgrown++] = m->ws;  // 1, 2, ... 32 MB: at most six
       m->ws = p;
       m->ws_bytes = bytes;
     }
     return RW_OK;
   }
   ~CallBuffer() {
+    if (own && p) cudaFreeAsync(p, m->st);
     cudaStreamSynchronize(m->st);  // nothing of the call is left on the buffer
-    if (own && p) cudaFree(p);
   }
 };
 
@@ -635,6 +641,7 @@ rw_status rw_mlp_destroy(rw_mlp* m) {
   for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->gord, (void*)m->m, (void*)m->v, (void*)m->fw, (void*)m->bw,
                   (void*)m->bias, (void*)m->err, (void*)m->loss, (void*)m->ranges, (void*)m->sx, (void*)m->stg, (void*)m->ws})
     if (p) cudaFree(p);
+  for (int k = 0; k < m->n_outgrown; ++k) cudaFree(m->outgrown[k]);
   if (m->st) cudaStreamDestroy(m->st);
   delete m;
   return RW_OK;
