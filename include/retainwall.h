@@ -320,7 +320,7 @@ rw_status rw_autotune(rw_ctx* ctx, int steps, int* chosen);
  * callers that cannot allocate device memory.  Stable sort of n cell keys (device
  * array d_keys, values in [0, max_key]) into d_sorted_keys, with d_perm[i] = index of
  * the key that lands at position i: the permutation NeighborSearch applies.  Uses a
- * fixed scratch array inside the library (8,913,924 bytes: 8.9 MB, 8.5 MiB, reserved
+ * fixed scratch array inside the library (8,913,920 bytes: 8.9 MB, 8.5 MiB, reserved
  * on every GPU that loads the library until the process exits) instead of
  * allocating: n is limited to
  * RW_NOALLOC_MAX_KEYS and max_key to 2^24 - 1 (RW_EINVAL beyond).  Runs on `stream`

@@ -616,7 +616,6 @@ template <class T> struct Engine final : EngineBase {
   }
   long beside_soil = 0, beside_bnd = 0;  // particles of the batch being captured (0: this case alone)
   // Soil candidate lists are kept only with the walk kernels.
-  // Soil candidate lists are kept only with the walk kernels.
   bool lists_kept() const { return ix_kernel == 0 && P.np > P.npb && S.nbg[0] && P.keep_lists; }
   void search(int section) {
     // Every kernel of the search returns at once when no particle changed cell since

@@ -3216,7 +3216,7 @@ static __global__ void k_wall_force_final(double* wsum, int nblocks) {
 
 // ---------------------------------------------------------------------------------
 // Export of arrays whose rows are not stored as the reference lays them out: element k of a
-// run of rows from `first`, written to page-locked host memory in order.
+// run of rows from `first`, written in order to the device buffer that is copied out.
 // ---------------------------------------------------------------------------------
 template <class T> struct Rows6 {
   const V4<T>* a;

@@ -18,14 +18,13 @@ namespace {
 constexpr int kMaxKeys = RW_NOALLOC_MAX_KEYS;
 constexpr int kMaxCounts = 256 * 512, kMaxBins = 256;
 
-// Scratch: ping-pong keys/values, per-tile digit counts, digit totals, sort flag:
-// 2 x 2^20 + 256 x 512 + 257 ints = 8,913,924 bytes (8.9 MB, 8.5 MiB).
+// Scratch: ping-pong keys/values, per-tile digit counts, digit totals:
+// 2 x 2^20 + 256 x 512 + 256 ints = 8,913,920 bytes (8.9 MB, 8.5 MiB).
 struct Scratch {
   int tk[kMaxKeys];
   int tv[kMaxKeys];
   int hist[kMaxCounts];
   int dtot[kMaxBins];
-  int spare;  // keeps the stated size
 };
 static __device__ __align__(256) Scratch g_scratch;
 
