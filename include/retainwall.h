@@ -356,9 +356,9 @@ rw_status rw_mlp_destroy(rw_mlp* m);
 rw_status rw_mlp_get_params(rw_mlp* m, float* out, size_t n);
 rw_status rw_mlp_set_params(rw_mlp* m, const float* in, size_t n);
 /* y[n][6] = net(x[n][16]).  The device copies of the host arrays of rw_mlp_forward and
- * rw_mlp_grad stay with the network until it is destroyed, up to 64 MB and at most as much again
- * in smaller ones of earlier calls (a call larger than any before allocates); a call that needs
- * more than 64 MB (762,600 samples) gives it back when it ends. */
+ * rw_mlp_grad (88 bytes a sample) stay with the network until it is destroyed: a buffer of up to
+ * 64 MB and the smaller ones it outgrew, together at most as much.  A call larger than any before
+ * allocates; one that fits no buffer to be kept gives its memory back when it ends. */
 rw_status rw_mlp_forward(rw_mlp* m, const float* x, int64_t n, float* y);
 /* Mean squared error over n samples and 6 outputs, and its gradient (RW_MLP_NPARAM). */
 rw_status rw_mlp_grad(rw_mlp* m, const float* x, const float* t, int64_t n, double* loss, float* grad);

@@ -441,15 +441,15 @@ struct rw_mlp {
   float* sx = nullptr;
   float* stg = nullptr;
   long long cap = 0, n = 0;
-  // Device copy of the host arrays of rw_mlp_forward / rw_mlp_grad, kept between calls up to
-  // kKeep bytes; more is allocated for the call, in stream order (given back to the driver at
-  // the wait: 0.2 to 2 ms a call, which is why smaller ones are kept).  Sizes are kFirst times a
-  // power of two, and outgrown buffers stay until the network goes: cudaFree waits for the work
-  // of every stream on the device.
-  static constexpr size_t kKeep = 64u << 20, kFirst = 1u << 20;
+  // Device copy of the host arrays of rw_mlp_forward / rw_mlp_grad, kept between calls.  A larger
+  // call gets a buffer at least twice as large, up to kKeep bytes; outgrown ones stay until the
+  // network goes, because cudaFree waits for the work of every stream on the device.  What fits
+  // neither is allocated for the call, in stream order (and given back to the driver at the
+  // wait: 0.2 to 2 ms a call, which is why smaller ones are kept).
+  static constexpr size_t kKeep = 64u << 20;
   unsigned char* ws = nullptr;
   size_t ws_bytes = 0;
-  void* outgrown[8] = {};
+  void* outgrown[32] = {};
   int n_outgrown = 0;
   std::string msg;
   std::mutex mu;
@@ -534,23 +534,19 @@ struct CallBuffer {
       p = m->ws;
       return RW_OK;
     }
-    own = bytes > rw_mlp::kKeep;
-    if (!own) {
-      size_t size = rw_mlp::kFirst;
-      while (size < bytes) size *= 2;
-      bytes = size;
-    }
+    const size_t grown = std::max(bytes, 2 * m->ws_bytes);
+    own = grown > rw_mlp::kKeep;
     const cudaError_t e = own ? cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, m->st)
-                              : cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+                              : cudaMalloc(reinterpret_cast<void**>(&p), grown);
     if (e != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
       return fail(m, RW_ECUDA, std::string("device memory of the call: ") + cudaGetErrorString(e));
     }
     if (!own) {
-      if (m->ws) m->outgrown[m->n_outgrown++] = m->ws;  // 1, 2, ... 32 MB: at most six
+      if (m->ws) m->outgrown[m->n_outgrown++] = m->ws;  // each twice the one before: fewer than 32
       m->ws = p;
-      m->ws_bytes = bytes;
+      m->ws_bytes = grown;
     }
     return RW_OK;
   }
