@@ -47,18 +47,18 @@ def metric_of(workload: str) -> str:
     """The headline metric for the 1.92M wall; the same quantity named for the other cases."""
     return METRICS.get(workload, METRIC)
 # From the ncu capture of the interaction's walk kernel on the 0.96M-particle case
-# (profiles/k_interaction_wall2_half.md): DRAM read+write 461.4 + 63.4 MB and 260M warp
+# (profiles/k_interaction_wall2_half.md): DRAM read+write 475.4 + 65.4 MB and 290M warp
 # instructions per launch.  Both grow with the particle count, so they are scaled per
 # soil particle to the benchmarked case.
-IX_DRAM_BYTES_PER_SOIL = (461.41e6 + 63.44e6) / 960000
-IX_WARP_INSTR_PER_SOIL = 260e6 / 960000
+IX_DRAM_BYTES_PER_SOIL = (475.44e6 + 65.36e6) / 960000
+IX_WARP_INSTR_PER_SOIL = 290.1e6 / 960000
 # L1 data-stage wavefronts the walk kernel cannot avoid: each listed neighbour's 64-byte
 # record is two 32-byte sectors read by one lane (records of a warp's lanes are distinct),
-# each list entry an eighth of a sector (a warp's 32 entries are one coalesced 128-byte
-# load), each particle's own state and outputs about 240 B.  The L1 data stage serves two
+# each list entry a quarter of a sector (a warp reads half a quad a lane, 8 of every 16
+# bytes: 16 sectors for 64 entries), each particle's own state and outputs about 240 B.  The L1 data stage serves two
 # scattered sectors per cycle per SM where they lie in different halves of a 64-byte
 # record, as odd and even lanes read them; a sector that is not in L1 costs a cycle more.
-IX_L1_SECTORS_PER_ENTRY = 2 + 1 / 8
+IX_L1_SECTORS_PER_ENTRY = 2 + 1 / 4
 IX_L1_SECTORS_PER_SOIL = 240 / 32
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # Host bytes rw_create_from_case copies per particle (int32 x4 codes, double x4 position,
@@ -594,7 +594,7 @@ def run_ours(args, ws, rank, local):
     roof_l1 = {"bound": "L1 data stage", "kernel": "k_interaction", "achieved": l1_sectors / (ix_ms * 1e-3),
                "peak": l1_peak, "unit": "sectors/s", "frac": l1_sectors / (ix_ms * 1e-3) / l1_peak,
                "sectors_per_launch": l1_sectors,
-               "note": "2 sectors per listed neighbour (64-B record) + 1/8 per list entry + 7.5 per particle; "
+               "note": "2 sectors per listed neighbour (64-B record) + 1/4 per list entry + 7.5 per particle; "
                        "sectors that miss L1 (about a quarter) cost a cycle more and are not counted"}
     line = {
         "metric": metric_of(args.workload), "value": value, "unit": "particle-updates/s", "n_gpus": ws,

@@ -124,8 +124,9 @@ typedef struct rw_info {
   double time, dt, h, dr;
   int32_t n_sorts;       /* neighbour-search sections whose sort permuted the particles     */
   int32_t n_list_reuse;  /* interactions that walked kept candidate lists                    */
-  int32_t n_search_skipped; /* gated searches (captured steps, and stage calls from a context's
-                               third step on) skipped whole (no particle changed cell)          */
+  int32_t n_search_skipped; /* gated searches (captured steps, and stage calls from a
+                               context's third step on while no option changes) skipped
+                               whole (no particle changed cell)                                 */
   int32_t n_scan_skipped;   /* captured-step interactions whose scan launch was skipped (every
                                particle walked a kept list)                                      */
   int32_t n_build_skipped;     /* gated searches whose list build was skipped (the kept lists
