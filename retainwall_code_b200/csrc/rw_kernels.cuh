@@ -1733,7 +1733,7 @@ RWD void load_half(const float* q, float (&v)[8]) {
 // after the other, so every sum is the one ix_list_eval forms, bit for bit.  Squares that
 // are then added stay scalar: the compiler fuses a packed multiply into a packed add.
 //
-// What bounds it: issue (half the cycles) and the L1 data stage (70% of its wavefronts)
+// What bounds it: issue (61% of the cycles) and the L1 data stage (78% of its wavefronts)
 // together.  The stage serves two lanes' 32-byte sectors per cycle when they lie in
 // different halves of a line's 64-byte half, one otherwise (measured on random records:
 // 51 cycles per warp and record pair of loads, 33 when odd lanes read the halves in the
@@ -1743,7 +1743,10 @@ RWD void load_half(const float* q, float (&v)[8]) {
 // rate.  1.92M-particle wall, per launch: 1.004 ms scalar, 0.955 ms packed with branches
 // around the sums, 0.909 ms with predicated sums and the flushing reciprocals, 0.882 ms with
 // the lists in quads (two entries a load, digits of the offset by a mask).  Scalar terms on
-// the same lists: 0.903 ms (122 registers), 0.937 ms at five blocks.
+// the same lists: 0.903 ms (122 registers), 0.937 ms at five blocks.  The viscous quotient is
+// divided with flushing first and again without where that is not normal, so that subnormal
+// ones are pair_eval's: 0.855 ms with and without; unflushed for every pair 0.878, one shared
+// branch for both pairs 0.960.
 RWD void ix_walk_pairs(const Params<float>& P, const DevState<float>& S, const IState<float>& I,
                        const unsigned* __restrict__ lists, int t_col, size_t stride, int cnt, Acc<float>& A) {
   if (cnt <= 0) return;
